@@ -7,7 +7,8 @@
 // the 48 KB static limit, and A = B = 64 does not compile) and the block size is
 // capped by the register file at large A.
 //
-// Here a CTA owns one channel f, a tile of TT = 4 TG consecutive time samples and
+// Here up to 16 beams run in the streaming kernel of beamform_stream.cuh.  For more a
+// CTA owns one channel f, a tile of TT = 4 TG consecutive time samples and
 // a tile of BT = 4 (256 / TG) beams.  Thread (tg, bg) accumulates a 4 x 4 register
 // tile: 4 consecutive time samples x 4 beams x P polarisations.  Antennas stream
 // through double-buffered shared memory in chunks of AC = 256 / TG (voltages stored
@@ -22,19 +23,13 @@
 // polarisations, and the integration window is closed with warp shuffles over
 // adjacent lanes.  Nothing but the Stokes-I output touches HBM.
 #include "autotune.cuh"
+#include "beamform_stream.cuh"
 #include "common.cuh"
 
 namespace bb {
 namespace {
 
 enum { IN_CF32 = 0, IN_CI8 = 1 };
-
-// Phasor element strides (float2 units) of beam, antenna, channel and
-// polarisation: [B, A, F, 1, P] for ATA, (A, 1, 0, 0) for MeerKAT's [B, A] weights
-// shared by every channel and polarisation.
-struct PhLayout {
-    uint64_t sb, sa, sf, sp;
-};
 
 inline PhLayout ata_layout(uint64_t A, uint64_t F, uint64_t P) { return PhLayout{A * F * P, F * P, P, 1}; }
 
@@ -294,34 +289,6 @@ __global__ void __launch_bounds__(256) incoherent_kernel(const float2* __restric
     }
 }
 
-// Small blocks (the tiled kernel would leave SMs idle): one thread per
-// (beam, channel, sample) and both polarisations, antennas in order; the CTA's
-// phasors are the same for all its threads and its voltages come from L2 (every
-// beam re-reads them).  Same arithmetic as the tiled kernel per output.
-template <int P>
-__global__ void __launch_bounds__(256) bf32_small_kernel(const float2* __restrict__ in,
-                                                         const float2* __restrict__ phasors, float2* __restrict__ out,
-                                                         uint32_t A, uint32_t F, uint32_t T, const PhLayout ph) {
-    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x, f = blockIdx.y, b = blockIdx.z;
-    if (t >= T) return;
-    float2 acc[P];
-#pragma unroll
-    for (int p = 0; p < P; p++) acc[p] = make_float2(0.f, 0.f);
-    const float2* x = in + ((uint64_t)f * T + t) * P;
-    const float2* w = phasors + b * ph.sb + (uint64_t)f * ph.sf;
-    for (uint32_t a = 0; a < A; a++) {
-#pragma unroll
-        for (int p = 0; p < P; p++) {
-            const float2 xv = __ldg(x + (uint64_t)a * F * T * P + p), wv = __ldg(w + a * ph.sa + p * ph.sp);
-            acc[p].x = fmaf(xv.x, wv.x, fmaf(-xv.y, wv.y, acc[p].x));
-            acc[p].y = fmaf(xv.x, wv.y, fmaf(xv.y, wv.x, acc[p].y));
-        }
-    }
-    float2* o = out + (((uint64_t)b * F + f) * T + t) * P;
-#pragma unroll
-    for (int p = 0; p < P; p++) o[p] = acc[p];
-}
-
 template <int P, int TG, int IN, int R>
 void launch_bf(const void* in, const float2* ph, void* out, uint64_t B, uint64_t A, uint64_t F, uint64_t T,
                uint64_t integ, cudaStream_t s, const PhLayout& lay) {
@@ -354,24 +321,57 @@ bool dims_ok(uint64_t B, uint64_t A, uint64_t F, uint64_t T) {
 namespace bb {
 namespace {
 
-// Beams 0..B-1 of the plain FP32 beamformer for a phasor layout (no incoherent beam).
+template <int P>
+int launch_stream_beams(const StreamArgs& g, uint32_t nb, uint32_t ns, cudaStream_t s) {
+#define BB_STREAM(NBV)                                                              \
+    (ns == 2 ? launch_stream<P, NBV, 2, STREAM_CF32, 0>(g, s) : launch_stream<P, NBV, 1, STREAM_CF32, 0>(g, s))
+    switch (nb) {
+        case 1: return BB_STREAM(1);
+        case 2: return BB_STREAM(2);
+        case 4: return BB_STREAM(4);
+        default: return BB_STREAM(8);
+    }
+#undef BB_STREAM
+}
+
+// Beams 0..B-1 of the plain FP32 beamformer for a phasor layout, and with inc the
+// incoherent beam of beam 0's weights (1 sum of powers, 2 its root).
 int beamform_f32_beams(const char* who, const void* in, const float2* ph, void* out, uint64_t B, uint64_t A,
-                       uint64_t F, uint64_t T, uint64_t P, const PhLayout& lay, cudaStream_t s) {
+                       uint64_t F, uint64_t T, uint64_t P, const PhLayout& lay, int inc, cudaStream_t s) {
     if (B == 0) return BLADE_SUCCESS;
     const int tg = pick_tg(B);
     const uint64_t tiles = ceil_div(T, (uint64_t)tg * 4) * F * ceil_div(B, (uint64_t)(256 / tg) * 4);
-    if (tiles < 2ull * sm_count() && B <= 65535) {
-        const dim3 grid((unsigned)ceil_div(T, 256), (unsigned)F, (unsigned)B);
+    // Up to 16 beams the voltages are read once or twice and the streaming kernel is
+    // faster at every size measured (1.2x at 16 beams, 1.8x at 8, 2.5x at one); with more
+    // it would read them once per eight beams, which only pays when the tiled kernel
+    // leaves SMs idle (64 beams x 64 antennas x 4 channels x 512 samples: 13.1 against
+    // 17.3 us for one thread per output).
+    uint32_t nb, ns;
+    if ((B <= 16 || tiles < 2ull * sm_count()) && stream_shape(B, A, F, T, P, nb, ns)) {
+        StreamArgs g{};
+        g.in = in;
+        g.ph = ph;
+        g.out = out;
+        g.B = (uint32_t)B;
+        g.A = (uint32_t)A;
+        g.F = (uint32_t)F;
+        g.T = (uint32_t)T;
+        g.inc = (uint32_t)inc;
+        g.lay = lay;
+        if (int rc = P == 2 ? launch_stream_beams<2>(g, nb, ns, s) : launch_stream_beams<1>(g, nb, ns, s)) return rc;
+        return check_launch(who);
+    }
+    if (P == 2) dispatch_tg<2, IN_CF32, 0>(tg, in, ph, out, B, A, F, T, 1, s, lay);
+    else dispatch_tg<1, IN_CF32, 0>(tg, in, ph, out, B, A, F, T, 1, s, lay);
+    if (inc) {
+        const float2* x = static_cast<const float2*>(in);
+        float2* y = static_cast<float2*>(out);
         if (P == 2)
-            bf32_small_kernel<2><<<grid, 256, 0, s>>>(static_cast<const float2*>(in), ph, static_cast<float2*>(out),
-                                                      (uint32_t)A, (uint32_t)F, (uint32_t)T, lay);
+            incoherent_kernel<2><<<grid_for(F * T, 256), 256, 0, s>>>(x, ph, y, (uint32_t)B, (uint32_t)A, (uint32_t)F,
+                                                                     (uint32_t)T, inc == 2);
         else
-            bf32_small_kernel<1><<<grid, 256, 0, s>>>(static_cast<const float2*>(in), ph, static_cast<float2*>(out),
-                                                      (uint32_t)A, (uint32_t)F, (uint32_t)T, lay);
-    } else if (P == 2) {
-        dispatch_tg<2, IN_CF32, 0>(tg, in, ph, out, B, A, F, T, 1, s, lay);
-    } else {
-        dispatch_tg<1, IN_CF32, 0>(tg, in, ph, out, B, A, F, T, 1, s, lay);
+            incoherent_kernel<1><<<grid_for(F * T, 256), 256, 0, s>>>(x, ph, y, (uint32_t)B, (uint32_t)A, (uint32_t)F,
+                                                                     (uint32_t)T, inc == 2);
     }
     return check_launch(who);
 }
@@ -399,21 +399,8 @@ extern "C" int blade_beamform_f32(const void* in, const void* phasors, void* out
     if (incoherent && B == 0) return set_error(BLADE_ERROR, "blade_beamform_f32: incoherent beam needs beam 0");
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
     const float2* ph = static_cast<const float2*>(phasors);
-    if (int rc = beamform_f32_beams("blade_beamform_f32", in, ph, out, B, A, F, T, P, ata_layout(A, F, P), s))
-        return rc;
-    if (incoherent) {
-        if (P == 2)
-            incoherent_kernel<2><<<grid_for(F * T, 256), 256, 0, s>>>(static_cast<const float2*>(in), ph,
-                                                                     static_cast<float2*>(out), (uint32_t)B,
-                                                                     (uint32_t)A, (uint32_t)F, (uint32_t)T,
-                                                                     incoherent_sqrt);
-        else
-            incoherent_kernel<1><<<grid_for(F * T, 256), 256, 0, s>>>(static_cast<const float2*>(in), ph,
-                                                                     static_cast<float2*>(out), (uint32_t)B,
-                                                                     (uint32_t)A, (uint32_t)F, (uint32_t)T,
-                                                                     incoherent_sqrt);
-    }
-    return check_launch("blade_beamform_f32");
+    return beamform_f32_beams("blade_beamform_f32", in, ph, out, B, A, F, T, P, ata_layout(A, F, P),
+                              incoherent ? (incoherent_sqrt ? 2 : 1) : 0, s);
 }
 
 extern "C" int blade_beamform_meerkat_f32(const void* in, const void* phasors, void* out, uint64_t B, uint64_t A,
@@ -424,7 +411,7 @@ extern "C" int blade_beamform_meerkat_f32(const void* in, const void* phasors, v
     if (int rc = check_f32_args("blade_beamform_meerkat_f32", in, phasors, out, B, A, F, T, P)) return rc;
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
     if (int rc = beamform_f32_beams("blade_beamform_meerkat_f32", in, static_cast<const float2*>(phasors), out, B, A,
-                                    F, T, P, PhLayout{A, 1, 0, 0}, s))
+                                    F, T, P, PhLayout{A, 1, 0, 0}, 0, s))
         return rc;
     if (incoherent) {
         // the reference sizes the incoherent beam but its MeerKAT kernel never writes it

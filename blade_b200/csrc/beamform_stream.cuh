@@ -1,0 +1,250 @@
+// Streaming FP32 beamformer for few beams: voltages go straight from global memory
+// to registers, once per tile of NB beams.
+//
+//   y[b, f, t, p] = sum_a x[a, f, t, p] w[b, a, f, 0, p]
+// (reference src/modules/beamformer/beamformer.cu:13-79), with the incoherent beam
+// sum_a |x w[0]|^2 from the same loads (beamformer.cu:64-78), stored as beam
+// voltages or, for Stokes-I and full-Stokes detection (detector.cu:7-51), as window
+// sums that never leave the registers as voltages.
+//
+// A warp owns 32 NS consecutive samples of one channel (lane l: samples l + 32 s)
+// and NB beams; a CTA's four warps take consecutive tiles, which may lie in up to
+// four channels when the channels are short.  Each antenna costs NS 16-byte loads
+// per lane (kU antennas in flight ahead of the arithmetic) and NB broadcast reads of
+// its weights from shared memory, which the NS samples share.
+//
+// Bound by the voltage read plus the FP32 pipe (57 % issue, long_scoreboard the
+// top stall): 20 antennas x 192 channels x 8192 samples, 8 beams: 163 us for 705 MB
+// (4.3 TB/s), where staging voltages and weights in shared memory took 288 us
+// behind its barriers (one every two antennas).  Packed FP32x2 arithmetic is no
+// faster (173 us), nor are one sample (165 us) or four beams x four samples (166 us)
+// per thread.
+#pragma once
+
+#include "common.cuh"
+
+namespace bb {
+
+// Phasor element strides (float2 units) of beam, antenna, channel and
+// polarisation: [B, A, F, 1, P] for ATA, (A, 1, 0, 0) for MeerKAT's [B, A] weights
+// shared by every channel and polarisation.
+struct PhLayout {
+    uint64_t sb, sa, sf, sp;
+};
+
+struct StreamArgs {
+    const void* in;
+    const float2* ph;
+    void* out;
+    uint32_t B, A, F, T;
+    uint32_t log_integ;  // detected outputs: window = 2^log_integ samples, at most 32
+    uint32_t inc;        // 0 none, 1 sum of powers, 2 its square root
+    uint32_t nbt;        // beam tiles, innermost in the grid (they read the same voltages)
+    uint32_t ntt;        // time tiles per channel
+    uint64_t tiles;      // F * ntt
+    PhLayout lay;
+};
+
+constexpr int kStreamWarps = 4;
+
+enum { STREAM_CF32 = 0, STREAM_CI8 = 1 };
+
+template <int P, int IN>
+__device__ __forceinline__ void stream_load(const void* in, uint64_t i, float2 (&v)[P]) {
+    if constexpr (IN == STREAM_CF32 && P == 2) {
+        const float4 q = ldg_nc_f4(static_cast<const float4*>(in) + i);
+        v[0] = make_float2(q.x, q.y);
+        v[1] = make_float2(q.z, q.w);
+    } else if constexpr (IN == STREAM_CF32) {
+        v[0] = __ldg(static_cast<const float2*>(in) + i);
+    } else if constexpr (P == 2) {
+        const char4 q = __ldg(static_cast<const char4*>(in) + i);
+        v[0] = make_float2((float)q.x, (float)q.y);
+        v[1] = make_float2((float)q.z, (float)q.w);
+    } else {
+        const char2 q = __ldg(static_cast<const char2*>(in) + i);
+        v[0] = make_float2((float)q.x, (float)q.y);
+    }
+}
+
+// OP = 0: beam voltages CF32 [B (+ 1), F, T, P]; OP = 1 or 4: detected products F32
+// [B (+ 1), F, T / I, OP] (P = 2).
+template <int P, int NB, int NS, int IN, int OP>
+__global__ void __launch_bounds__(kStreamWarps * 32, NB == 8 && NS == 2 ? 4 : 1) bf_stream_kernel(const StreamArgs g) {
+    constexpr int kU = 4 / NS;  // antennas per load round, two rounds in flight
+    extern __shared__ __align__(16) float2 ws[];  // [channel][A padded to kU][NB][P]
+    const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+    const uint32_t Ap = (g.A + kU - 1) / kU * kU;
+    const uint32_t blk = blockIdx.x / g.nbt, b0 = (blockIdx.x - blk * g.nbt) * NB;
+    const uint64_t first = (uint64_t)blk * kStreamWarps;
+    const uint64_t last = min(first + kStreamWarps, g.tiles) - 1;
+    const uint32_t f0 = (uint32_t)(first / g.ntt), nch = (uint32_t)(last / g.ntt) - f0 + 1;
+    // weights of this CTA's channels, padded beams and antennas zero
+    for (uint32_t r = tid; r < NB * Ap; r += kStreamWarps * 32) {
+        const uint32_t a = r / NB, j = r - a * NB;
+        const bool ok = a < g.A && b0 + j < g.B;
+        const float2* src = g.ph + (b0 + j) * g.lay.sb + a * g.lay.sa + (uint64_t)f0 * g.lay.sf;
+        for (uint32_t c = 0; c < nch; c++)
+#pragma unroll
+            for (int p = 0; p < P; p++)
+                ws[((c * Ap + a) * NB + j) * P + p] = ok ? __ldg(src + c * g.lay.sf + p * g.lay.sp) : make_float2(0.f, 0.f);
+    }
+    __syncthreads();
+    const uint64_t tile = first + warp;
+    if (tile > last) return;
+    const uint32_t f = (uint32_t)(tile / g.ntt), t0 = (uint32_t)(tile - (uint64_t)f * g.ntt) * (32 * NS) + lane;
+    const uint64_t astride = (uint64_t)g.F * g.T, x0 = (uint64_t)f * g.T + t0;
+    const float2* wc = ws + (size_t)(f - f0) * Ap * NB * P;
+    const bool inc = g.inc != 0 && b0 == 0;
+
+    float2 acc[NB][NS][P];
+    float pw[NS][P];
+#pragma unroll
+    for (int s = 0; s < NS; s++)
+#pragma unroll
+        for (int p = 0; p < P; p++) {
+            pw[s][p] = 0.f;
+#pragma unroll
+            for (int j = 0; j < NB; j++) acc[j][s][p] = make_float2(0.f, 0.f);
+        }
+    auto load = [&](uint32_t a0, float2 (&x)[kU][NS][P]) {
+#pragma unroll
+        for (int u = 0; u < kU; u++)
+#pragma unroll
+            for (int s = 0; s < NS; s++) {
+                if (a0 + u < g.A && t0 + 32 * s < g.T) {
+                    stream_load<P, IN>(g.in, (a0 + u) * astride + x0 + 32 * s, x[u][s]);
+                } else {
+#pragma unroll
+                    for (int p = 0; p < P; p++) x[u][s][p] = make_float2(0.f, 0.f);
+                }
+            }
+    };
+    auto mac = [&](uint32_t a0, const float2 (&x)[kU][NS][P]) {
+#pragma unroll
+        for (int u = 0; u < kU; u++) {
+            const float2* wa = wc + (size_t)(a0 + u) * NB * P;
+#pragma unroll
+            for (int j = 0; j < NB; j++) {
+                float2 w[P];
+                if constexpr (P == 2) {
+                    const float4 q = *reinterpret_cast<const float4*>(wa + j * P);
+                    w[0] = make_float2(q.x, q.y);
+                    w[1] = make_float2(q.z, q.w);
+                } else {
+                    w[0] = wa[j];
+                }
+#pragma unroll
+                for (int s = 0; s < NS; s++)
+#pragma unroll
+                    for (int p = 0; p < P; p++) {
+                        const float2 xv = x[u][s][p];
+                        acc[j][s][p].x = fmaf(xv.x, w[p].x, fmaf(-xv.y, w[p].y, acc[j][s][p].x));
+                        acc[j][s][p].y = fmaf(xv.x, w[p].y, fmaf(xv.y, w[p].x, acc[j][s][p].y));
+                        if (j == 0 && inc) {
+                            const float re = xv.x * w[p].x - xv.y * w[p].y, im = xv.x * w[p].y + xv.y * w[p].x;
+                            pw[s][p] += re * re + im * im;
+                        }
+                    }
+            }
+        }
+    };
+    float2 xa[kU][NS][P], xb[kU][NS][P];
+    load(0, xa);
+#pragma unroll 1
+    for (uint32_t a0 = 0; a0 < g.A; a0 += 2 * kU) {
+        if (a0 + kU < g.A) load(a0 + kU, xb);
+        mac(a0, xa);
+        if (a0 + kU >= g.A) break;
+        if (a0 + 2 * kU < g.A) load(a0 + 2 * kU, xa);
+        mac(a0 + kU, xb);
+    }
+
+    if constexpr (OP == 0) {
+        float2* out = static_cast<float2*>(g.out);
+#pragma unroll
+        for (int s = 0; s < NS; s++) {
+            if (t0 + 32 * s >= g.T) continue;
+#pragma unroll
+            for (int j = 0; j < NB; j++) {
+                if (b0 + j >= g.B) continue;
+                float2* o = out + ((b0 + j) * astride + x0 + 32 * s) * P;
+                if constexpr (P == 2) stg_f4(o, make_float4(acc[j][s][0].x, acc[j][s][0].y, acc[j][s][1].x, acc[j][s][1].y));
+                else o[0] = acc[j][s][0];
+            }
+            if (inc) {
+                float2* o = out + (g.B * astride + x0 + 32 * s) * P;
+#pragma unroll
+                for (int p = 0; p < P; p++) o[p] = make_float2(g.inc == 2 ? sqrtf(pw[s][p]) : pw[s][p], 0.f);
+            }
+        }
+    } else if constexpr (P == 2) {
+        float* out = static_cast<float*>(g.out);
+        const uint32_t I = 1u << g.log_integ, U = g.T >> g.log_integ;
+        auto emit = [&](uint32_t row, int s, float2 x, float2 y) {
+            float v[OP];
+            if constexpr (OP == 1) {
+                v[0] = x.x * x.x + x.y * x.y + (y.x * y.x + y.y * y.y);
+            } else {
+                v[0] = x.x * x.x + x.y * x.y;
+                v[1] = y.x * y.x + y.y * y.y;
+                v[2] = x.x * y.x + x.y * y.y;  // Re x conj(y)
+                v[3] = x.y * y.x - x.x * y.y;  // Im x conj(y)
+            }
+            for (uint32_t o = 1; o < I; o <<= 1)
+#pragma unroll
+                for (int q = 0; q < OP; q++) v[q] += __shfl_xor_sync(0xffffffffu, v[q], o);
+            if ((lane & (I - 1u)) == 0 && t0 + 32 * s < g.T) {
+                float* d = out + (((uint64_t)row * g.F + f) * U + ((t0 + 32 * s) >> g.log_integ)) * OP;
+                if constexpr (OP == 4) stg_f4(d, make_float4(v[0], v[1], v[2], v[3]));
+                else d[0] = v[0];
+            }
+        };
+#pragma unroll
+        for (int s = 0; s < NS; s++) {
+#pragma unroll
+            for (int j = 0; j < NB; j++)
+                if (b0 + j < g.B) emit(b0 + j, s, acc[j][s][0], acc[j][s][1]);
+            if (inc) emit(g.B, s, make_float2(g.inc == 2 ? sqrtf(pw[s][0]) : pw[s][0], 0.f),
+                          make_float2(g.inc == 2 ? sqrtf(pw[s][1]) : pw[s][1], 0.f));
+        }
+    }
+}
+
+inline size_t stream_smem(uint64_t nb, uint64_t ns, uint64_t A, uint64_t F, uint64_t T, uint64_t P) {
+    const uint64_t kU = 4 / ns, Ap = (A + kU - 1) / kU * kU, ntt = ceil_div(T, 32 * ns);
+    // channels that a CTA's consecutive tiles can touch
+    uint64_t nch = ntt % kStreamWarps == 0 ? 1 : 1 + ceil_div(kStreamWarps - 1, ntt);
+    if (nch > F) nch = F;
+    return nch * Ap * nb * P * sizeof(float2);
+}
+
+// Beams and samples per thread.  Eight beams share each voltage load and two samples
+// each weight read as long as every SM still gets eight warps; below that, fewer, so
+// that a small block spreads over the SMs (20 antennas x 96 channels x 256 samples,
+// 8 beams with the incoherent beam: 8.8 us against 17.3 us for one thread per
+// output).  False: the weights do not fit in shared memory.
+inline bool stream_shape(uint64_t B, uint64_t A, uint64_t F, uint64_t T, uint64_t P, uint32_t& nb, uint32_t& ns) {
+    nb = B > 4 ? 8 : B > 2 ? 4 : (uint32_t)B;
+    ns = 2;
+    const uint64_t want = 8ull * sm_count();
+    if (F * ceil_div(T, 64) * ceil_div(B, nb) < want) ns = 1;
+    while (nb > 2 && F * ceil_div(T, 32 * ns) * ceil_div(B, nb) < want) nb /= 2;
+    while (nb > 1 && stream_smem(nb, ns, A, F, T, P) > 160 * 1024) nb /= 2;
+    return stream_smem(nb, ns, A, F, T, P) <= 160 * 1024 &&
+           ceil_div(F * ceil_div(T, 32 * ns), kStreamWarps) * ceil_div(B, nb) < (1ull << 31);
+}
+
+template <int P, int NB, int NS, int IN, int OP>
+int launch_stream(StreamArgs g, cudaStream_t s) {
+    g.ntt = (uint32_t)ceil_div(g.T, 32 * NS);
+    g.tiles = (uint64_t)g.F * g.ntt;
+    g.nbt = (uint32_t)ceil_div(g.B, NB);
+    const size_t smem = stream_smem(NB, NS, g.A, g.F, g.T, P);
+    const auto fn = bf_stream_kernel<P, NB, NS, IN, OP>;
+    if (int rc = ensure_smem(reinterpret_cast<const void*>(fn), smem)) return rc;
+    fn<<<(unsigned)(ceil_div(g.tiles, kStreamWarps) * g.nbt), kStreamWarps * 32, smem, s>>>(g);
+    return BLADE_SUCCESS;
+}
+
+}  // namespace bb
