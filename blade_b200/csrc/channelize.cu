@@ -9,15 +9,18 @@
 // tests/modules/channelizer/advanced.py:49-65:
 //   out[a, f*C + k, s, p] = fftshift(FFT_C(x[a, f, s*C:(s+1)*C, p]))[k].
 //
-// Here, rate <= 4096: one CTA loads whole spectra of one (a, f) (all
-// polarisations) with coalesced loads into shared memory, runs mixed-radix
-// Stockham passes (radix 8/4/2 and direct odd-prime DFTs, twiddles from a
-// shared-memory table computed with sincospif) and writes the spectra transposed
-// into the [A, F*C, T/C, P] layout with the fftshift folded into the store index.
+// Here, rates 2 to 16 (powers of two) hold one spectrum per thread in registers and
+// powers of two from 32 to 4096 run in fft_pow2.cu.  Other rates <= 4096: one CTA
+// loads whole spectra of one (a, f) (all polarisations) with coalesced loads into
+// shared memory, runs mixed-radix Stockham passes (radix 8/4/2 and direct odd-prime
+// DFTs, twiddles from a shared-memory table computed with sincospif) and writes the
+// spectra transposed into the [A, F*C, T/C, P] layout with the fftshift folded into
+// the store index.
 // rate > 4096: a four-step FFT (C = N1 * N2): column FFTs of length N1 with the
 // inter-step twiddle, written to a workspace, then row FFTs of length N2 written
 // to the output.
 #include "autotune.cuh"
+#include "channelize.cuh"
 #include "common.cuh"
 #include "tc_ptx.cuh"
 
@@ -870,6 +873,7 @@ extern "C" int blade_channelize(const void* in, void* out, void* workspace, uint
 #undef BB_FFT_REG
         return check_launch("blade_channelize");
     }
+    if (channelize_pow2_applies(rate)) return channelize_pow2(src, false, dst, A, F, T, P, rate, 0, s);
     if (rate <= kSmallMax) {
         Plan plan;
         if (!make_plan(rate, plan))
