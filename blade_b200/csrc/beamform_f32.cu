@@ -403,6 +403,80 @@ extern "C" int blade_beamform_f32(const void* in, const void* phasors, void* out
                               incoherent ? (incoherent_sqrt ? 2 : 1) : 0, s);
 }
 
+namespace bb {
+namespace {
+
+// Whether the beams and the incoherent beam run through the detector inside the
+// streaming kernel: windows that a warp closes with lane shuffles, and at most two
+// reads of the voltages (16 beams, 28 antennas x 768 channels x 2048 samples: 467 us
+// against 735 us for the kernels one by one; 8 beams x 20 antennas 1.7 to 2.5 times
+// faster; beyond 16 beams the tiled beamformer reads the voltages less often).
+bool products_shape(uint64_t B, uint64_t A, uint64_t F, uint64_t T, uint64_t P, uint64_t I, uint64_t out_pols,
+                    uint32_t& nb) {
+    uint32_t ns;
+    if (P != 2 || B == 0 || B > 16 || A == 0 || F == 0 || T == 0 || !dims_ok(B, A, F, T)) return false;
+    if (I == 0 || I > 32 || (I & (I - 1)) != 0 || T % I != 0 || (out_pols != 1 && out_pols != 4)) return false;
+    // one sample per thread: the products' shuffles need the registers of the second
+    return stream_shape(B, A, F, T, P, nb, ns) && stream_smem(nb, 1, A, F, T, P) <= 160 * 1024 &&
+           ceil_div(F * ceil_div(T, 32), kStreamWarps) * ceil_div(B, nb) < (1ull << 31);
+}
+
+template <int IN, int OP>
+int launch_products(const StreamArgs& g, uint32_t nb, cudaStream_t s) {
+    switch (nb) {
+        case 1: return launch_stream<2, 1, 1, IN, OP>(g, s);
+        case 2: return launch_stream<2, 2, 1, IN, OP>(g, s);
+        case 4: return launch_stream<2, 4, 1, IN, OP>(g, s);
+        default: return launch_stream<2, 8, 1, IN, OP>(g, s);
+    }
+}
+
+}  // namespace
+}  // namespace bb
+
+extern "C" int blade_beamform_products_supported(uint64_t B, uint64_t A, uint64_t F, uint64_t T, uint64_t P,
+                                                 uint64_t integration, uint64_t out_pols) {
+    uint32_t nb;
+    return bb::products_shape(B, A, F, T, P, integration, out_pols, nb) ? 1 : 0;
+}
+
+extern "C" int blade_beamform_products_f32(int in_type, const void* in, const void* phasors, void* out, uint64_t B,
+                                           uint64_t A, uint64_t F, uint64_t T, uint64_t P, uint64_t integration,
+                                           uint64_t out_pols, int incoherent, blade_stream_t stream) {
+    using namespace bb;
+    const char* who = "blade_beamform_products_f32";
+    if (in_type != BLADE_CF32 && in_type != BLADE_CI8)
+        return set_error(BLADE_ERROR, "%s: input type must be CF32 or CI8", who);
+    uint32_t nb;
+    if (!products_shape(B, A, F, T, P, integration, out_pols, nb))
+        return set_error(BLADE_ERROR,
+                         "%s: unsupported configuration (B=%llu A=%llu F=%llu T=%llu P=%llu I=%llu out_pols=%llu): "
+                         "needs P = 2, 1 <= B <= 16, I a power of two <= 32 dividing T, 1 or 4 products", who,
+                         (unsigned long long)B, (unsigned long long)A, (unsigned long long)F, (unsigned long long)T,
+                         (unsigned long long)P, (unsigned long long)integration, (unsigned long long)out_pols);
+    if (!in || !phasors || !out) return set_error(BLADE_ERROR, "%s: null buffer", who);
+    if ((reinterpret_cast<uintptr_t>(in) & (in_type == BLADE_CF32 ? 15 : 3)) ||
+        (reinterpret_cast<uintptr_t>(out) & (out_pols == 4 ? 15 : 3)))
+        return set_error(BLADE_ERROR, "%s: misaligned buffer", who);
+    StreamArgs g{};
+    g.in = in;
+    g.ph = static_cast<const float2*>(phasors);
+    g.out = out;
+    g.B = (uint32_t)B;
+    g.A = (uint32_t)A;
+    g.F = (uint32_t)F;
+    g.T = (uint32_t)T;
+    while ((1ull << g.log_integ) < integration) g.log_integ++;
+    g.inc = incoherent ? 2 : 0;
+    g.lay = ata_layout(A, F, P);
+    cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+    int rc;
+    if (in_type == BLADE_CF32) rc = out_pols == 1 ? launch_products<STREAM_CF32, 1>(g, nb, s)
+                                                  : launch_products<STREAM_CF32, 4>(g, nb, s);
+    else rc = out_pols == 1 ? launch_products<STREAM_CI8, 1>(g, nb, s) : launch_products<STREAM_CI8, 4>(g, nb, s);
+    return rc ? rc : check_launch(who);
+}
+
 extern "C" int blade_beamform_meerkat_f32(const void* in, const void* phasors, void* out, uint64_t B, uint64_t A,
                                           uint64_t F, uint64_t T, uint64_t P, int incoherent, blade_stream_t stream) {
     using namespace bb;

@@ -18,7 +18,9 @@
 // (4.3 TB/s), where staging voltages and weights in shared memory took 288 us
 // behind its barriers (one every two antennas).  Packed FP32x2 arithmetic is no
 // faster (173 us), nor are one sample (165 us) or four beams x four samples (166 us)
-// per thread.
+// per thread.  With detection (20 antennas x 6144 channels x 128 samples, 8 beams and
+// the incoherent one, four products): 105 us against 470 us for the tiled kernel,
+// the incoherent kernel and the detector.
 #pragma once
 
 #include "common.cuh"
@@ -57,13 +59,11 @@ __device__ __forceinline__ void stream_load(const void* in, uint64_t i, float2 (
         v[1] = make_float2(q.z, q.w);
     } else if constexpr (IN == STREAM_CF32) {
         v[0] = __ldg(static_cast<const float2*>(in) + i);
-    } else if constexpr (P == 2) {
-        const char4 q = __ldg(static_cast<const char4*>(in) + i);
-        v[0] = make_float2((float)q.x, (float)q.y);
-        v[1] = make_float2((float)q.z, (float)q.w);
     } else {
-        const char2 q = __ldg(static_cast<const char2*>(in) + i);
-        v[0] = make_float2((float)q.x, (float)q.y);
+        static_assert(P == 2, "CI8 input is dual-polarisation");
+        const float4 q = ci8_f4(__ldg(static_cast<const uint32_t*>(in) + i));
+        v[0] = make_float2(q.x, q.y);
+        v[1] = make_float2(q.z, q.w);
     }
 }
 
@@ -79,34 +79,11 @@ __global__ void __launch_bounds__(kStreamWarps * 32, NB == 8 && NS == 2 ? 4 : 1)
     const uint64_t first = (uint64_t)blk * kStreamWarps;
     const uint64_t last = min(first + kStreamWarps, g.tiles) - 1;
     const uint32_t f0 = (uint32_t)(first / g.ntt), nch = (uint32_t)(last / g.ntt) - f0 + 1;
-    // weights of this CTA's channels, padded beams and antennas zero
-    for (uint32_t r = tid; r < NB * Ap; r += kStreamWarps * 32) {
-        const uint32_t a = r / NB, j = r - a * NB;
-        const bool ok = a < g.A && b0 + j < g.B;
-        const float2* src = g.ph + (b0 + j) * g.lay.sb + a * g.lay.sa + (uint64_t)f0 * g.lay.sf;
-        for (uint32_t c = 0; c < nch; c++)
-#pragma unroll
-            for (int p = 0; p < P; p++)
-                ws[((c * Ap + a) * NB + j) * P + p] = ok ? __ldg(src + c * g.lay.sf + p * g.lay.sp) : make_float2(0.f, 0.f);
-    }
-    __syncthreads();
     const uint64_t tile = first + warp;
-    if (tile > last) return;
-    const uint32_t f = (uint32_t)(tile / g.ntt), t0 = (uint32_t)(tile - (uint64_t)f * g.ntt) * (32 * NS) + lane;
+    const bool active = tile <= last;
+    const uint32_t f = active ? (uint32_t)(tile / g.ntt) : f0;
+    const uint32_t t0 = (uint32_t)(tile - (uint64_t)f * g.ntt) * (32 * NS) + lane;
     const uint64_t astride = (uint64_t)g.F * g.T, x0 = (uint64_t)f * g.T + t0;
-    const float2* wc = ws + (size_t)(f - f0) * Ap * NB * P;
-    const bool inc = g.inc != 0 && b0 == 0;
-
-    float2 acc[NB][NS][P];
-    float pw[NS][P];
-#pragma unroll
-    for (int s = 0; s < NS; s++)
-#pragma unroll
-        for (int p = 0; p < P; p++) {
-            pw[s][p] = 0.f;
-#pragma unroll
-            for (int j = 0; j < NB; j++) acc[j][s][p] = make_float2(0.f, 0.f);
-        }
     auto load = [&](uint32_t a0, float2 (&x)[kU][NS][P]) {
 #pragma unroll
         for (int u = 0; u < kU; u++)
@@ -120,6 +97,35 @@ __global__ void __launch_bounds__(kStreamWarps * 32, NB == 8 && NS == 2 ? 4 : 1)
                 }
             }
     };
+    float2 xa[kU][NS][P], xb[kU][NS][P];
+    // on their way while the weights are gathered (with two samples per thread the
+    // registers held across the gather cost more: 170 against 163 us on the block above)
+    if (NS == 1 && active) load(0, xa);
+    // weights of this CTA's channels, padded beams and antennas zero
+    for (uint32_t r = tid; r < NB * Ap; r += kStreamWarps * 32) {
+        const uint32_t a = r / NB, j = r - a * NB;
+        const bool ok = a < g.A && b0 + j < g.B;
+        const float2* src = g.ph + (b0 + j) * g.lay.sb + a * g.lay.sa + (uint64_t)f0 * g.lay.sf;
+        for (uint32_t c = 0; c < nch; c++)
+#pragma unroll
+            for (int p = 0; p < P; p++)
+                ws[((c * Ap + a) * NB + j) * P + p] = ok ? __ldg(src + c * g.lay.sf + p * g.lay.sp) : make_float2(0.f, 0.f);
+    }
+    __syncthreads();
+    if (!active) return;
+    const float2* wc = ws + (size_t)(f - f0) * Ap * NB * P;
+    const bool inc = g.inc != 0 && b0 == 0;
+
+    float2 acc[NB][NS][P];
+    float pw[NS][P];
+#pragma unroll
+    for (int s = 0; s < NS; s++)
+#pragma unroll
+        for (int p = 0; p < P; p++) {
+            pw[s][p] = 0.f;
+#pragma unroll
+            for (int j = 0; j < NB; j++) acc[j][s][p] = make_float2(0.f, 0.f);
+        }
     auto mac = [&](uint32_t a0, const float2 (&x)[kU][NS][P]) {
 #pragma unroll
         for (int u = 0; u < kU; u++) {
@@ -149,8 +155,7 @@ __global__ void __launch_bounds__(kStreamWarps * 32, NB == 8 && NS == 2 ? 4 : 1)
             }
         }
     };
-    float2 xa[kU][NS][P], xb[kU][NS][P];
-    load(0, xa);
+    if (NS != 1) load(0, xa);
 #pragma unroll 1
     for (uint32_t a0 = 0; a0 < g.A; a0 += 2 * kU) {
         if (a0 + kU < g.A) load(a0 + kU, xb);

@@ -83,6 +83,17 @@ __device__ __forceinline__ uint4 ldg_nc_u4(const void* p) {
     return v;
 }
 
+// The four int8 of a word as floats: byte b ^ 0x80 in the low mantissa bits of 2^23 is
+// 2^23 + 128 + b, and the subtraction is exact.  (The convert instruction issues at a
+// quarter of this rate.)
+__device__ __forceinline__ float4 ci8_f4(uint32_t w) {
+    const uint32_t x = w ^ 0x80808080u;
+    return make_float4(__uint_as_float(__byte_perm(x, 0x4B000000u, 0x7650)) - 8388736.f,
+                       __uint_as_float(__byte_perm(x, 0x4B000000u, 0x7651)) - 8388736.f,
+                       __uint_as_float(__byte_perm(x, 0x4B000000u, 0x7652)) - 8388736.f,
+                       __uint_as_float(__byte_perm(x, 0x4B000000u, 0x7653)) - 8388736.f);
+}
+
 __device__ __forceinline__ void stg_f4(void* p, float4 v) {
     *reinterpret_cast<float4*>(p) = v;
 }

@@ -113,8 +113,7 @@ __device__ __forceinline__ c2 pair(float4 q) { return {make_float2(q.x, q.z), ma
 
 // One dual-polarisation CI8 sample [p0 re, p0 im, p1 re, p1 im], exact
 __device__ __forceinline__ c2 pair_ci8(uint32_t w) {
-    return {make_float2((float)(int8_t)(w & 0xFFu), (float)(int8_t)((w >> 16) & 0xFFu)),
-            make_float2((float)(int8_t)((w >> 8) & 0xFFu), (float)(int8_t)(w >> 24))};
+    return pair(ci8_f4(w));
 }
 
 // The pair as consecutive complex values; circular != 0: (X + iY, X - iY)

@@ -914,6 +914,66 @@ class _ModeBTensorCore(Module):
         return result.success
 
 
+class _ModeBPre(Module):
+    """Cast -> Channelizer -> [Polarizer] of ModeB in one launch
+    (blade_prechannelize_cf32), into a buffer of its own."""
+
+    taint = Taint.CONSUMER | Taint.PRODUCER
+
+    def __init__(self, buffer, rate, circular):
+        super().__init__()
+        self._buffer, self._R, self._circ = buffer, int(rate), bool(circular)
+        A, F, T, P = as_vector(buffer).shape
+        self._output = self._alloc((A, F * self._R, T // self._R, P), "cf32")
+
+    @staticmethod
+    def applies(it, T, P, R) -> bool:
+        # on CF32 the Channelizer at rate T and the Polarizer at rate 1 work in the
+        # caller's buffer, as the reference's do: those stay with the modules
+        if P != 2 or R < 1 or R > 4096 or T % R or (R % 2 and R != 1):
+            return False
+        return it == "ci8" or R not in (1, T)
+
+    def get_output(self):
+        return self._output
+
+    def process(self, step=0, stream=None):
+        x, out = as_vector(self._buffer), _out(self._output)
+        A, F, T, P = x.shape
+        _lib.call("blade_prechannelize_cf32", type_code(x.dtype), x.data_ptr(), out.data_ptr(), A, F, T, P, self._R,
+                  int(self._circ), _stream_handle(stream))
+        return result.success
+
+
+class _BeamformProducts(Module):
+    """Beamformer (+ square-rooted incoherent beam) -> Detector in one launch
+    (blade_beamform_products_f32): the beams never reach memory as voltages."""
+
+    taint = Taint.CONSUMER | Taint.PRODUCER
+
+    def __init__(self, buffer, phasors, integration, out_pols, incoherent):
+        super().__init__()
+        self._buffer, self._phasors = buffer, phasors
+        self._I, self._OP, self._inc = int(integration), int(out_pols), bool(incoherent)
+        A, F, T, P = as_vector(buffer).shape
+        B = as_vector(phasors).shape[0]
+        self._output = self._alloc((B + int(self._inc), F, T // self._I, self._OP), "f32")
+
+    @staticmethod
+    def applies(A, F, T, P, B, I, OP) -> bool:
+        return I > 0 and _lib.load().blade_beamform_products_supported(B, A, F, T, P, I, OP) == 1
+
+    def get_output(self):
+        return self._output
+
+    def process(self, step=0, stream=None):
+        x, ph, out = as_vector(self._buffer), as_vector(self._phasors), _out(self._output)
+        A, F, T, P = x.shape
+        _lib.call("blade_beamform_products_f32", type_code(x.dtype), x.data_ptr(), ph.data_ptr(), out.data_ptr(),
+                  ph.shape[0], A, F, T, P, self._I, self._OP, int(self._inc), _stream_handle(stream))
+        return result.success
+
+
 class ModeB(Module):
     """Bundles::ATA::ModeB<IT, OT> (include/blade/bundles/ata/mode_b.hh:17-225, Python
     binding python/blade/ext_modeb.cc:20-114): Cast -> Channelizer (pre-beamformer,
@@ -933,8 +993,10 @@ class ModeB(Module):
     as one fused launch (tensor cores for CI8 input, FP32 CUDA cores for CF32).
     CI8 input at rate 2 or 4 with Stokes-I runs the pre-beamformer stages into
     exact FP16 and the tensor-core chain on the fine channels, plus the detected
-    incoherent beam when enabled (``tensor_cores`` is True); every other
-    configuration runs the module kernels in order."""
+    incoherent beam when enabled (``tensor_cores`` is True).  Elsewhere the
+    pre-beamformer stages run as one launch up to rate 4096, and up to 16 beams the
+    Beamformer -> Detector pair as another (windows of up to 32 spectra, a power of
+    two); what these do not take runs the module kernels in order."""
 
     taint = Taint.CONSUMER | Taint.PRODUCER
 
@@ -1021,18 +1083,30 @@ class ModeB(Module):
                                   BeamformDetect.input(buffer=input.buffer, phasors=phasors), it=it, ot="f32")
             self._stages.append(last)
         else:
-            cast = Cast(Cast.config(c.cast_block_size), Cast.input(input.buffer), it=it, ot="cf32")
-            chan = Channelizer(Channelizer.config(R, c.channelizer_block_size), Channelizer.input(cast.get_output()))
-            polz = Polarizer(Polarizer.config(pol.xy, pol.lr if c.pre_beamformer_polarizer_convert_to_circular
-                                              else pol.xy, c.polarizer_block_size),
-                             Polarizer.input(chan.get_output()))
-            bf = BeamformerATA(BeamformerATA.config(bool(c.beamformer_incoherent_beam), bool(c.detector_enable),
-                                                    c.beamformer_block_size),
-                               BeamformerATA.input(polz.get_output(), phasors))
-            self._stages += [cast, chan, polz, bf]
-            last = bf
-            if c.detector_enable:
-                last = Detector(Detector.config(I, OP, c.detector_block_size), Detector.input(bf.get_output()))
+            circ, inc = bool(c.pre_beamformer_polarizer_convert_to_circular), bool(c.beamformer_incoherent_beam)
+            products = (bool(c.detector_enable) and OP in (1, 4) and R >= 1 and T % R == 0
+                        and _BeamformProducts.applies(A, F * R, T // R, P, B, I, OP))
+            if R == 1 and not circ and P == 2 and (products or it == "cf32"):
+                voltages = input.buffer
+            elif _ModeBPre.applies(it, T, P, R):
+                pre = _ModeBPre(input.buffer, R, circ)
+                voltages = pre.get_output()
+                self._stages.append(pre)
+            else:
+                cast = Cast(Cast.config(c.cast_block_size), Cast.input(input.buffer), it=it, ot="cf32")
+                chan = Channelizer(Channelizer.config(R, c.channelizer_block_size), Channelizer.input(cast.get_output()))
+                polz = Polarizer(Polarizer.config(pol.xy, pol.lr if circ else pol.xy, c.polarizer_block_size),
+                                 Polarizer.input(chan.get_output()))
+                voltages = polz.get_output()
+                self._stages += [cast, chan, polz]
+            if products:
+                last = _BeamformProducts(voltages, phasors, I, OP, inc)
+            else:
+                last = BeamformerATA(BeamformerATA.config(inc, bool(c.detector_enable), c.beamformer_block_size),
+                                     BeamformerATA.input(voltages, phasors))
+            self._stages.append(last)
+            if c.detector_enable and not products:
+                last = Detector(Detector.config(I, OP, c.detector_block_size), Detector.input(last.get_output()))
                 self._stages.append(last)
         self._last = last
         out_shape = tuple(as_vector(last.get_output()).shape)

@@ -112,6 +112,24 @@ BLADE_API int blade_beamform_meerkat_f32(const void* in, const void* phasors, vo
                                uint64_t P, int incoherent, blade_stream_t stream);
 
 /* ---------------------------------------------------------------------------
+ * Beamformer::ATA (with its square-rooted incoherent beam when incoherent != 0)
+ * followed by the Detector, in one pass over the voltages:
+ *   out F32 [B+inc, F, T/I, out_pols] = blade_detect(blade_beamform_f32(in, ..., sqrt))
+ * in: CF32 or CI8 (cast exactly) [A,F,T,2]; phasors: CF32 [B,A,F,1,2]; out_pols 1 or 4.
+ * Limits (blade_beamform_products_supported() returns 1 when met): P = 2,
+ * 1 <= B <= 16, I a power of two <= 32 dividing T, and the weights of a few beams
+ * in shared memory (A up to a few hundred).
+ * Composes src/modules/beamformer/beamformer.cu:13-79 and src/modules/detector/
+ * detector.cu:7-51 as Bundles::ATA::ModeB chains them (mode_b.hh:146-199).
+ * ------------------------------------------------------------------------- */
+BLADE_API int blade_beamform_products_supported(uint64_t B, uint64_t A, uint64_t F, uint64_t T,
+                                      uint64_t P, uint64_t integration, uint64_t out_pols);
+BLADE_API int blade_beamform_products_f32(int in_type, const void* in, const void* phasors,
+                                void* out, uint64_t B, uint64_t A, uint64_t F, uint64_t T,
+                                uint64_t P, uint64_t integration, uint64_t out_pols,
+                                int incoherent, blade_stream_t stream);
+
+/* ---------------------------------------------------------------------------
  * Channelizer: [A,F,T,P] CF32 -> [A,F*rate,T/rate,P] CF32,
  *   out[a, f*rate + k, s, p] = fftshift(FFT_rate(in[a, f, s*rate:(s+1)*rate, p]))[k]
  * unnormalised, hand-written FP32 Stockham FFT.  rate = 1 copies (or is a no-op
@@ -128,6 +146,18 @@ BLADE_API uint64_t blade_channelize_workspace_size(uint64_t A, uint64_t F, uint6
 BLADE_API int blade_channelize(const void* in, void* out, void* workspace,
                      uint64_t A, uint64_t F, uint64_t T, uint64_t P, uint64_t rate,
                      blade_stream_t stream);
+
+/* ---------------------------------------------------------------------------
+ * Cast -> Channelizer(rate) -> [Polarizer] in one pass, the pre-beamformer stages of
+ * Bundles::ATA::ModeB (include/blade/bundles/ata/mode_b.hh:99-139): CI8 or CF32
+ * [A,F,T,2] in, CF32 [A, F*rate, T/rate, 2] out, (X, Y) -> (X + iY, X - iY) when
+ * circular != 0.  Same values as blade_cast, blade_channelize and blade_polarize.
+ * rate 1 or an even rate <= 4096 dividing T with prime factors <= 61 (P must be 2);
+ * in and out must not overlap.
+ * ------------------------------------------------------------------------- */
+BLADE_API int blade_prechannelize_cf32(int in_type, const void* in, void* out, uint64_t A,
+                             uint64_t F, uint64_t T, uint64_t P, uint64_t rate,
+                             int circular, blade_stream_t stream);
 
 /* ---------------------------------------------------------------------------
  * Fused spectrometer: Cast -> Channelizer(rate) -> Polarizer -> Detector ->
