@@ -22,6 +22,7 @@
 #include "autotune.cuh"
 #include "channelize.cuh"
 #include "common.cuh"
+#include "fft_regs.cuh"
 #include "tc_ptx.cuh"
 
 namespace bb {
@@ -557,290 +558,249 @@ __global__ void __launch_bounds__(256, 2) fft8192_kernel(const float2* __restric
     }
 }
 
-// Column step for N = 65536 (N1 = N2 = 256): one CTA = one (a, f, s) spectrum, 16
-// consecutive columns j2, both polarisations (32 FFTs x 16 threads = 512 threads).
-// Output ws[((batch P + p) 256 + k1) 256 + j2] = w65536^(j2 k1) FFT256_j1(x[256 j1 + j2])[k1].
-// Padded stride of a 256-point column / row in shared memory: odd, so columns
-// read or written side by side fall in different banks, and >= 16 * 17 so the
-// 16 x 16 exchange can use row stride 17 (conflict-free in both directions).
-constexpr uint32_t kLd = 273;
-constexpr uint32_t kZ = 17;
+// ---- rate 65536 = 256 x 256 on pairs of transforms (fft_regs.cuh) ------------
+// n = j2 + 256 j1, k = k1 + 256 k2:
+//   W[k1][j2] = sum_j1 x[j2 + 256 j1] w256^(j1 k1)                    (column step)
+//   X[k]      = sum_j2 w65536^(j2 k1) W[k1][j2] w256^(j2 k2)          (row step)
+// Each 256-point transform runs on 16 threads as 16 x 16 with one shared-memory
+// exchange of 16-byte pairs; both steps load their inputs straight into registers
+// and store their results from them.  A unit is a spectrum of both polarisations, or
+// two consecutive spectra of a single one; ws holds W as pairs (re of both members,
+// im of both members), [(a, f)][unit][k1][j2], so the row step needs no re-pairing.
+// The inter-step twiddles sit in the row step, whose CTA needs 256 of them per k1 for
+// all its units: each is one sincospif, rounded once.
+//
+// Bound by HBM behind the workspace round trip: the spectrometer's 64 channels x 16
+// spectra (CI8 in, windows of 8) 531 us for 2.45 GB (4.6 TB/s), 796 us for one
+// transform per thread group with three shared-memory passes per step and twiddle
+// recurrences.  The next group's input is asked for while a group is transformed (551 us
+// without); three CTAs per SM spill and take 730 us.  Error against 64 bits 1.5e-7
+// where the recurrences gave 4.2e-7.
+constexpr uint32_t k65Threads = 256;
+constexpr uint32_t k65Ld = 257;  // pairs per unit in the row step's exchange
 
-// v[k] *= w^k for k = 0..15 by recurrence from w (15 complex products, relative
-// error a few FP32 ulps): replaces 16 strided, bank-conflicting table lookups.
-__device__ __forceinline__ void twiddle_run(float2 (&v)[16], float2 base, float2 w) {
-    float2 acc = base;
-#pragma unroll
-    for (int k = 0; k < 16; k++) {
-        v[k] = cmul(v[k], acc);
-        acc = cmul(acc, w);
-    }
+// The last row of w256^(t k), k = 1 .. 15, t < 16, is at tw[14 * 16].
+__device__ __forceinline__ void fill_w256(float2* tw) {
+    for (uint32_t i = threadIdx.x; i < 15 * 16; i += blockDim.x) tw[i] = fft::root((i / 16 + 1) * (i % 16), 256);
 }
 
-// CI8 = true: the input is CI8 [.., T, 2] (one 4-byte word per dual-polarisation
-// sample), cast exactly to FP32 on load (the fused spectrometer).
-template <int P, bool CI8 = false>
-__global__ void __launch_bounds__(512, 2) fft256_cols_kernel(const void* __restrict__ vin, float2* __restrict__ ws,
-                                                          uint64_t batches) {
-    extern __shared__ __align__(16) float2 sm[];
-    float2* tile = sm;                   // [p][jc][kLd]   (16 P columns)
-    float2* w256 = tile + 16 * P * kLd;  // w256^m, m < 256
-    float2* wlo = w256 + 256;            // w65536^m, m < 256
-    for (uint32_t m = threadIdx.x; m < 256; m += blockDim.x) {
-        w256[m] = twiddle(m, 256);
-        wlo[m] = twiddle(m, 65536);
-    }
-    const uint32_t t = threadIdx.x & 15u, jc = (threadIdx.x >> 4) & 15u, p = threadIdx.x >> 8;
-    const bool active = p < (uint32_t)P;
-    float2* col = tile + (p * 16 + jc) * kLd;
-    constexpr uint32_t kPer = 256u * 16u / 512u;  // words loaded per thread per group
-    // CI8: the next group's words are loaded into registers while this group's FFTs
-    // run (8 registers), so the loads of consecutive groups overlap the arithmetic.
-    uint32_t nxt[kPer];
-    auto load_ci8 = [&](uint64_t g, uint32_t (&w)[kPer]) {
-        const uint32_t* src = static_cast<const uint32_t*>(vin) + (g >> 4) * 65536ull + (uint32_t)(g & 15u) * 16u;
+// Column step: one CTA = 16 columns j2 of one unit.  Thread (t, jc) loads rows
+// j1 = 16 m + t (consecutive threads, consecutive columns); ex[(t 16 + k) 16 + jc]
+// keeps the columns innermost, so every access is conflict-free.
+template <int P, bool CI8>
+__global__ void __launch_bounds__(k65Threads, 2) fft256_cols_kernel(const void* __restrict__ vin,
+                                                                    float4* __restrict__ ws, uint64_t rows,
+                                                                    uint32_t S) {
+    extern __shared__ __align__(16) float4 ex[];                       // [16][16][16]
+    float2* tw = reinterpret_cast<float2*>(ex + 4096);                 // w256^(t k)
+    fill_w256(tw);
+    __syncthreads();
+    const uint32_t jc = threadIdx.x & 15u, t = threadIdx.x >> 4;
+    const uint32_t Su = P == 2 ? S : (S + 1) / 2;
+    const uint64_t groups = rows * Su * 16;
+    // CI8: the next group's words travel while this group is transformed (16
+    // registers); wider inputs are asked into L2 instead
+    uint32_t nxt[CI8 ? 16 : 1];
+    auto load_ci8 = [&](uint64_t g) {
+        const uint32_t* src = static_cast<const uint32_t*>(vin) + (g >> 4) * 65536ull + t * 256u + (uint32_t)(g & 15u) * 16u + jc;
 #pragma unroll
-        for (uint32_t u = 0; u < kPer; u++) {
-            const uint32_t e = threadIdx.x + u * 512u;
-            w[u] = __ldg(src + (uint64_t)(e >> 4) * 256u + (e & 15u));
-        }
+        for (int m = 0; m < (CI8 ? 16 : 1); m++) nxt[m] = __ldg(src + m * 4096);
     };
     if constexpr (CI8)
-        if (blockIdx.x < batches * 16) load_ci8(blockIdx.x, nxt);
-    for (uint64_t grp = blockIdx.x; grp < batches * 16; grp += gridDim.x) {
-        const uint64_t batch = grp >> 4;
-        const uint32_t c0 = (uint32_t)(grp & 15u) * 16u;
-        __syncthreads();
-        // coalesced load: rows j1 of 16 columns x P (256 B per row for P = 2); all of a
-        // thread's loads are issued before any shared-memory store
+        if (blockIdx.x < groups) load_ci8(blockIdx.x);
+    for (uint64_t grp = blockIdx.x; grp < groups; grp += gridDim.x) {
+        const uint64_t unit = grp >> 4;  // (a, f) row x Su + unit of the row
+        const uint32_t j2 = (uint32_t)(grp & 15u) * 16u + jc;
+        fft::c2 v[16];
         if constexpr (CI8) {
-            uint32_t ld[kPer];
 #pragma unroll
-            for (uint32_t u = 0; u < kPer; u++) ld[u] = nxt[u];
-            if (grp + gridDim.x < batches * 16) load_ci8(grp + gridDim.x, nxt);
+            for (int m = 0; m < 16; m++) v[m] = fft::pair_ci8(nxt[m]);
+            if (grp + gridDim.x < groups) load_ci8(grp + gridDim.x);
+        } else if constexpr (P == 2) {
+            const uint64_t base = unit * 65536ull + t * 256u + j2;
 #pragma unroll
-            for (uint32_t u = 0; u < kPer; u++) {
-                const uint32_t e = threadIdx.x + u * 512u, j1 = e >> 4, jl = e & 15u;
-                const uint32_t w = ld[u];
-                tile[(0 * 16 + jl) * kLd + j1] = make_float2((float)(int8_t)(w & 0xFFu), (float)(int8_t)((w >> 8) & 0xFFu));
-                tile[(1 * 16 + jl) * kLd + j1] = make_float2((float)(int8_t)((w >> 16) & 0xFFu), (float)(int8_t)(w >> 24));
-            }
-        } else if (P == 2) {
-            const float2* src = static_cast<const float2*>(vin) + batch * 65536ull * P;
-#pragma unroll
-            for (uint32_t h = 0; h < 2; h++) {  // two batches of four 16-byte loads in flight
-                float4 ld[kPer / 2];
-#pragma unroll
-                for (uint32_t u = 0; u < kPer / 2; u++) {
-                    const uint32_t e = threadIdx.x + (h * kPer / 2 + u) * 512u, j1 = e >> 4, jl = e & 15u;
-                    ld[u] = ldg_nc_f4(src + 2 * ((uint64_t)j1 * 256u + c0 + jl));
-                }
-#pragma unroll
-                for (uint32_t u = 0; u < kPer / 2; u++) {
-                    const uint32_t e = threadIdx.x + (h * kPer / 2 + u) * 512u, j1 = e >> 4, jl = e & 15u;
-                    tile[(0 * 16 + jl) * kLd + j1] = make_float2(ld[u].x, ld[u].y);
-                    tile[(1 * 16 + jl) * kLd + j1] = make_float2(ld[u].z, ld[u].w);
-                }
+            for (int m = 0; m < 16; m++) v[m] = fft::pair(ldg_nc_f4(static_cast<const float4*>(vin) + base + m * 4096));
+            if (grp + gridDim.x < groups) {  // row threadIdx.x of the next group: two 128-byte lines
+                const uint64_t g = grp + gridDim.x;
+                const float4* next = static_cast<const float4*>(vin) + (g >> 4) * 65536ull + threadIdx.x * 256u + (uint32_t)(g & 15u) * 16u;
+                tc::prefetch_l2(next);
+                tc::prefetch_l2(next + 8);
             }
         } else {
-            const float2* src = static_cast<const float2*>(vin) + batch * 65536ull * P;
-            float2 ld[kPer];
+            const uint64_t af = unit / Su;
+            const uint32_t s = 2 * (uint32_t)(unit - af * Su);
+            const float2* src = static_cast<const float2*>(vin) + (af * S + s) * 65536ull + t * 256u + j2;
+            const bool two = s + 1 < S;
 #pragma unroll
-            for (uint32_t u = 0; u < kPer; u++) {
-                const uint32_t e = threadIdx.x + u * 512u, j1 = e >> 4, jl = e & 15u;
-                ld[u] = src[(uint64_t)j1 * 256u + c0 + jl];
-            }
-#pragma unroll
-            for (uint32_t u = 0; u < kPer; u++) {
-                const uint32_t e = threadIdx.x + u * 512u, j1 = e >> 4, jl = e & 15u;
-                tile[jl * kLd + j1] = ld[u];
+            for (int m = 0; m < 16; m++) {
+                const float2 x = __ldg(src + m * 4096), y = two ? __ldg(src + 65536 + m * 4096) : make_float2(0.f, 0.f);
+                v[m] = fft::c2{make_float2(x.x, y.x), make_float2(x.y, y.y)};
             }
         }
-        __syncthreads();
-        float2 v[16];
-        if (active) {
+        fft::dft<16>(v);
+        fft::twiddle_column<16>(v, tw + t, 16);
 #pragma unroll
-            for (int n1 = 0; n1 < 16; n1++) v[n1] = col[16 * n1 + t];  // thread n2 = t
-            dft16(v);
-            twiddle_run(v, make_float2(1.f, 0.f), w256[t]);  // w256^(t k1)
-        }
+        for (int k = 0; k < 16; k++) ex[(t * 16 + k) * 16 + jc] = make_float4(v[k].re.x, v[k].re.y, v[k].im.x, v[k].im.y);
         __syncthreads();
-        if (active) {
 #pragma unroll
-            for (int k1 = 0; k1 < 16; k1++) col[kZ * t + k1] = v[k1];  // Z[n2 = t][k1]
+        for (int i = 0; i < 16; i++) {
+            const float4 q = ex[(i * 16 + t) * 16 + jc];
+            v[i] = fft::c2{make_float2(q.x, q.y), make_float2(q.z, q.w)};
         }
         __syncthreads();
-        if (active) {
+        fft::dft<16>(v);
+        float4* dst = ws + unit * 65536ull + t * 256u + j2;  // k1 = t + 16 k
 #pragma unroll
-            for (int n2 = 0; n2 < 16; n2++) v[n2] = col[kZ * n2 + t];  // thread k1 = t
-            dft16(v);  // X[t + 16 k2]
-            // inter-step twiddle w65536^(j2 (t + 16 k2)): base w^(j2 t), step w^(16 j2),
-            // each from the two-level table w256^(m >> 8) w65536^(m & 255)
-            const uint32_t j2 = c0 + jc;
-            const uint32_t m0 = j2 * t, m1 = (16u * j2) & 65535u;
-            twiddle_run(v, cmul(w256[m0 >> 8], wlo[m0 & 255u]), cmul(w256[m1 >> 8], wlo[m1 & 255u]));
-        }
-        __syncthreads();
-        if (active) {
-#pragma unroll
-            for (int k2 = 0; k2 < 16; k2++) col[t + 16 * k2] = v[k2];  // col[k1] = result, k1 = t + 16 k2
-        }
-        __syncthreads();
-        // coalesced store: for each (p, k1), 16 consecutive j2
-        for (uint32_t e = threadIdx.x; e < (uint32_t)P * 256u * 16u; e += blockDim.x) {
-            const uint32_t jl = e & 15u, k1 = (e >> 4) & 255u, pp = e >> 12;
-            ws[((batch * P + pp) * 256u + k1) * 256ull + c0 + jl] = tile[(pp * 16 + jl) * kLd + k1];
-        }
+        for (int k = 0; k < 16; k++) dst[k * 4096] = make_float4(v[k].re.x, v[k].re.y, v[k].im.x, v[k].im.y);
     }
 }
 
-// Loads the rows (s, p, k1) of one (a, f) for all S spectra x P polarisations
-// (q = s * P + p < nq) from the workspace into shared memory: 256 contiguous values
-// per row.
-__device__ __forceinline__ void load_rows(const float2* __restrict__ ws, float2* rows, uint64_t af, uint32_t S,
-                                          uint32_t P, uint32_t k1, uint32_t nq) {
-    // Asynchronous 8-byte copies straight into shared memory: all of a group's loads
-    // are in flight at once without holding registers (rows are 273 float2 apart, so
-    // 8 bytes is the widest aligned copy); consecutive threads take consecutive j2.
-    const uint32_t n = nq * 256u;
-    for (uint32_t e = threadIdx.x; e < n; e += blockDim.x) {
-        const uint32_t qq = e >> 8, j2 = e & 255u;
-        const float2* src = ws + (((af * S) * P + qq) * 256u + k1) * 256ull + j2;
-        const uint32_t dst = static_cast<uint32_t>(__cvta_generic_to_shared(rows + qq * kLd + j2));
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst), "l"(src) : "memory");
-    }
-    asm volatile("cp.async.wait_all;" ::: "memory");
-}
-
-// Row step for N = 65536: one CTA = one (a, f) and one k1, all S spectra x P
-// polarisations (S P <= 32 FFTs, 16 threads each).  X[k1 + 256 k2] goes to the
-// fftshifted channel k1 + 256 k2 + N/2 (mod N) of [A, F*N, S, P].
-template <int P>
-__global__ void __launch_bounds__(512, 2) fft256_rows_kernel(const float2* __restrict__ ws, float2* __restrict__ out,
-                                                          uint64_t AF, uint32_t S) {
-    extern __shared__ __align__(16) float2 sm[];
-    float2* rows = sm;                     // [q = s P + p][kLd], q < S P <= 32
-    float2* w256 = rows + 32 * kLd;
-    for (uint32_t m = threadIdx.x; m < 256; m += blockDim.x) w256[m] = twiddle(m, 256);
-    const uint32_t t = threadIdx.x & 15u, q = threadIdx.x >> 4;
-    const uint32_t nq = S * P;
-    const bool active = q < nq;
-    float2* row = rows + q * kLd;
-    for (uint64_t grp = blockIdx.x; grp < AF * 256u; grp += gridDim.x) {
-        const uint64_t af = grp >> 8;
-        const uint32_t k1 = (uint32_t)(grp & 255u);
-        __syncthreads();
-        load_rows(ws, rows, af, S, P, k1, nq);
-        __syncthreads();
-        float2 v[16];
-        if (active) {
+// Row step: one CTA = kk consecutive k1 of one (a, f), all its Su units (q = kk index x
+// Su + unit, kk Su <= 16).  OP = 0 stores the fftshifted spectra [A, F N, S, P]: the
+// values of a bin block (kk bins x S spectra x P) are contiguous.  OP = 1, 4 (P = 2)
+// stores the detector products of windows of I spectra, [A, F N, S / I, OP]: each
+// thread's products go through shared memory once and are summed over the window in
+// spectrum order.
+template <int P, int OP, typename OT>
+__global__ void __launch_bounds__(k65Threads, 2) fft256_rows_kernel(const float4* __restrict__ ws, void* __restrict__ vout,
+                                                                    uint64_t rows, uint32_t S, uint32_t kk, uint32_t I,
+                                                                    int circular) {
+    extern __shared__ __align__(16) float4 ex[];                 // [16 units][k65Ld]
+    float2* tw = reinterpret_cast<float2*>(ex + 16 * k65Ld);     // w256^(t k)
+    float2* tj = tw + 240;                                       // w65536^(k1 j2), [kk][256]
+    fill_w256(tw);
+    const uint32_t Su = P == 2 ? S : (S + 1) / 2;
+    const uint32_t nk = 256u / kk, Q = kk * Su;
+    const uint32_t lt = threadIdx.x & 15u, lq = threadIdx.x >> 4;  // load: 16 consecutive j2 per unit
+    const uint32_t lki = lq / Su;
+    for (uint64_t grp = blockIdx.x; grp < rows * nk; grp += gridDim.x) {
+        const uint64_t af = grp / nk;
+        const uint32_t kb = (uint32_t)(grp - af * nk) * kk;
+        fft::c2 v[16];
+        if (lq < Q) {
+            const float4* src = ws + ((af * Su + (lq - lki * Su)) * 256u + kb + lki) * 256ull + lt;
 #pragma unroll
-            for (int n1 = 0; n1 < 16; n1++) v[n1] = row[16 * n1 + t];
-            dft16(v);
-            twiddle_run(v, make_float2(1.f, 0.f), w256[t]);
+            for (int m = 0; m < 16; m++) {
+                const float4 q = __ldg(src + 16 * m);
+                v[m] = fft::c2{make_float2(q.x, q.y), make_float2(q.z, q.w)};
+            }
+            if (grp + gridDim.x < rows * nk) {  // the next group's 4 KB of this unit: two 128-byte lines per thread
+                const uint64_t g = grp + gridDim.x, naf = g / nk;
+                const uint32_t nkb = (uint32_t)(g - naf * nk) * kk;
+                const float4* next = ws + ((naf * Su + (lq - lki * Su)) * 256u + nkb + lki) * 256ull + lt * 8;
+                tc::prefetch_l2(next);
+                tc::prefetch_l2(next + 128);
+            }
+        }
+        for (uint32_t i = threadIdx.x; i < kk * 256u; i += k65Threads) tj[i] = fft::root((kb + (i >> 8)) * (i & 255u), 65536);
+        __syncthreads();
+        if (lq < Q) {
+#pragma unroll
+            for (int m = 0; m < 16; m++) v[m] = fft::mul(v[m], tj[lki * 256u + 16 * m + lt]);
+            fft::dft<16>(v);
+            fft::twiddle_column<16>(v, tw + lt, 16);
+#pragma unroll
+            for (int k = 0; k < 16; k++)
+                ex[lq * k65Ld + k * 16 + lt] = make_float4(v[k].re.x, v[k].re.y, v[k].im.x, v[k].im.y);
         }
         __syncthreads();
-        if (active) {
+        // thread (q, k): consecutive threads, consecutive units
+        const uint32_t q = threadIdx.x & 15u, k = threadIdx.x >> 4;
+        if (q < Q) {
 #pragma unroll
-            for (int k = 0; k < 16; k++) row[kZ * t + k] = v[k];
+            for (int i = 0; i < 16; i++) {
+                const float4 x = ex[q * k65Ld + k * 16 + i];
+                v[i] = fft::c2{make_float2(x.x, x.y), make_float2(x.z, x.w)};
+            }
+            fft::dft<16>(v);  // X[kb + ki + 256 (k + 16 m)]
         }
-        __syncthreads();
-        if (active) {
+        if constexpr (OP == 0) {
+            float2* out = static_cast<float2*>(vout);
+            if (q < Q) {
 #pragma unroll
-            for (int n2 = 0; n2 < 16; n2++) v[n2] = row[kZ * n2 + t];
-            dft16(v);  // X2[t + 16 c] = final X[k1 + 256 (t + 16 c)]
-        }
-        __syncthreads();
-        if (active) {
-#pragma unroll
-            for (int c = 0; c < 16; c++) row[t + 16 * c] = v[c];
-        }
-        __syncthreads();
-        // out[(af N + kout) S + s][p], kout = (k1 + 256 k2 + 32768) mod 65536; (s, p) fastest
-        for (uint32_t e = threadIdx.x; e < 256u * nq; e += blockDim.x) {
-            const uint32_t qq = e % nq, k2 = e / nq;
-            const uint32_t kout = (k1 + 256u * k2 + 32768u) & 65535u;
-            out[((af * 65536ull + kout) * S) * P + qq] = rows[qq * kLd + k2];
-        }
-    }
-}
-
-// Row step of the fused spectrometer: the row FFTs of fft256_rows_kernel, then
-// per output channel the optional circular conversion (L, R) = (X + iY, X - iY)
-// (Polarizer), the detector over windows of I spectra (Stokes-I |X|^2 + |Y|^2, or
-// (|X|^2, |Y|^2, Re X conj Y, Im X conj Y)) and the output cast, straight to
-// out[A, F*N, S/I, OP]: only the products reach HBM.
-template <int OP, typename OT>
-__global__ void __launch_bounds__(512, 2) fft256_rows_detect_kernel(const float2* __restrict__ ws, OT* __restrict__ out,
-                                                                 uint64_t AF, uint32_t S, uint32_t I, int circular) {
-    extern __shared__ __align__(16) float2 sm[];
-    constexpr uint32_t P = 2;
-    float2* rows = sm;  // [q = s P + p][kLd], q < S P <= 32
-    float2* w256 = rows + 32 * kLd;
-    for (uint32_t m = threadIdx.x; m < 256; m += blockDim.x) w256[m] = twiddle(m, 256);
-    const uint32_t t = threadIdx.x & 15u, q = threadIdx.x >> 4;
-    const uint32_t nq = S * P, U = S / I;
-    const bool active = q < nq;
-    float2* row = rows + q * kLd;
-    for (uint64_t grp = blockIdx.x; grp < AF * 256u; grp += gridDim.x) {
-        const uint64_t af = grp >> 8;
-        const uint32_t k1 = (uint32_t)(grp & 255u);
-        __syncthreads();
-        load_rows(ws, rows, af, S, P, k1, nq);
-        __syncthreads();
-        float2 v[16];
-        if (active) {
-#pragma unroll
-            for (int n1 = 0; n1 < 16; n1++) v[n1] = row[16 * n1 + t];
-            dft16(v);
-            twiddle_run(v, make_float2(1.f, 0.f), w256[t]);
-        }
-        __syncthreads();
-        if (active) {
-#pragma unroll
-            for (int k = 0; k < 16; k++) row[kZ * t + k] = v[k];
-        }
-        __syncthreads();
-        if (active) {
-#pragma unroll
-            for (int n2 = 0; n2 < 16; n2++) v[n2] = row[kZ * n2 + t];
-            dft16(v);
-        }
-        __syncthreads();
-        if (active) {
-#pragma unroll
-            for (int c = 0; c < 16; c++) row[t + 16 * c] = v[c];
-        }
-        __syncthreads();
-        // one thread per (k2, u): window sum over I spectra, OP products
-        for (uint32_t e = threadIdx.x; e < 256u * U; e += blockDim.x) {
-            const uint32_t u = e % U, k2 = e / U;
-            float acc[OP];
-#pragma unroll
-            for (int o = 0; o < OP; o++) acc[o] = 0.f;
-            for (uint32_t s = u * I; s < (u + 1) * I; s++) {
-                float2 x = rows[(s * 2 + 0) * kLd + k2], y = rows[(s * 2 + 1) * kLd + k2];
-                if (circular) {
-                    const float2 l = make_float2(x.x - y.y, x.y + y.x), r = make_float2(x.x + y.y, x.y - y.x);
-                    x = l;
-                    y = r;
-                }
-                if constexpr (OP == 1) {
-                    acc[0] += x.x * x.x + x.y * x.y + y.x * y.x + y.y * y.y;
-                } else {
-                    acc[0] += x.x * x.x + x.y * x.y;
-                    acc[1] += y.x * y.x + y.y * y.y;
-                    acc[2] += x.x * y.x + x.y * y.y;  // Re x conj(y)
-                    acc[3] += x.y * y.x - x.x * y.y;  // Im x conj(y)
+                for (int m = 0; m < 16; m++) {
+                    const uint32_t k0 = (kb + 256u * (k + 16u * m) + 32768u) & 65535u;  // fftshifted bin of ki = 0
+                    if constexpr (P == 2) {
+                        stg_f4(out + ((af * 65536ull + k0) * S + q) * 2, fft::unpair(v[m], 0));
+                    } else {
+                        const uint32_t ki = q / Su, s = 2 * (q - ki * Su);
+                        float2* dst = out + (af * 65536ull + k0 + ki) * S + s;
+                        if ((S & 1u) == 0) {
+                            stg_f4(dst, fft::unpair(v[m], 0));
+                        } else {
+                            dst[0] = make_float2(v[m].re.x, v[m].im.x);
+                            if (s + 1 < S) dst[1] = make_float2(v[m].re.y, v[m].im.y);
+                        }
+                    }
                 }
             }
-            const uint32_t kout = (k1 + 256u * k2 + 32768u) & 65535u;
-            OT* dst = out + ((af * 65536ull + kout) * U + u) * OP;
+            __syncthreads();  // the exchange and the twiddles are read before the next group writes them
+        } else {
+            __syncthreads();  // every unit has read its exchange words: products take their place
+            float* pw = reinterpret_cast<float*>(ex);  // [q][k65Ld][OP]
+            if (q < Q) {
 #pragma unroll
-            for (int o = 0; o < OP; o++) dst[o] = (OT)acc[o];
+                for (int m = 0; m < 16; m++) {
+                    const float4 x = fft::unpair(v[m], circular);
+                    float* d = pw + (q * k65Ld + k + 16 * m) * OP;
+                    if constexpr (OP == 1) {
+                        d[0] = x.x * x.x + x.y * x.y + x.z * x.z + x.w * x.w;
+                    } else {
+                        *reinterpret_cast<float4*>(d) =
+                            make_float4(x.x * x.x + x.y * x.y, x.z * x.z + x.w * x.w, x.x * x.z + x.y * x.w,
+                                        x.y * x.z - x.x * x.w);  // |x|^2, |y|^2, Re and Im of x conj(y)
+                    }
+                }
+            }
+            __syncthreads();
+            OT* out = static_cast<OT*>(vout);
+            const uint32_t U = S / I;
+            const uint32_t KU = kk * U;  // windows of a bin block, contiguous in the output
+            for (uint32_t e = threadIdx.x; e < 256u * KU; e += k65Threads) {
+                const uint32_t k2 = e / KU, w = e - k2 * KU, ki = w / U, u = w - ki * U;
+                float acc[OP];
+#pragma unroll
+                for (int o = 0; o < OP; o++) acc[o] = 0.f;
+                for (uint32_t i = 0; i < I; i++) {
+                    const float* d = pw + ((ki * S + u * I + i) * k65Ld + k2) * OP;
+                    if constexpr (OP == 1) {
+                        acc[0] += d[0];
+                    } else {
+                        const float4 x = *reinterpret_cast<const float4*>(d);
+                        acc[0] += x.x;
+                        acc[1] += x.y;
+                        acc[2] += x.z;
+                        acc[3] += x.w;
+                    }
+                }
+                const uint32_t kout = (kb + ki + 256u * k2 + 32768u) & 65535u;
+                OT* dst = out + ((af * 65536ull + kout) * U + u) * OP;
+                bool whole = false;
+                if constexpr (OP == 4 && sizeof(OT) == 4) {
+                    whole = (reinterpret_cast<uintptr_t>(vout) & 15u) == 0;
+                    if (whole) stg_f4(dst, make_float4(acc[0], acc[1], acc[2], acc[3]));
+                }
+                if (!whole) {
+#pragma unroll
+                    for (int o = 0; o < OP; o++) dst[o] = (OT)acc[o];
+                }
+            }
+            __syncthreads();
         }
     }
 }
+
+constexpr size_t k65ColsSmem = 4096 * sizeof(float4) + 240 * sizeof(float2);
+
+// Consecutive k1 per CTA of the row step: the largest power of two with at most 16
+// units, so that short blocks still store whole sectors.
+inline uint32_t rows_kk(uint32_t Su) {
+    uint32_t kk = 1;
+    while (2 * kk * Su <= 16) kk *= 2;
+    return kk;
+}
+
+inline size_t rows_smem(uint32_t kk) { return 16 * k65Ld * sizeof(float4) + (240 + 256 * kk) * sizeof(float2); }
 
 template <typename K>
 int prepare_smem(K kernel, size_t bytes) {
@@ -914,6 +874,8 @@ bool split_large(uint64_t N, uint64_t& N1, uint64_t& N2) {
 
 extern "C" uint64_t blade_channelize_workspace_size(uint64_t A, uint64_t F, uint64_t T, uint64_t P, uint64_t rate) {
     if (rate <= bb::kSmallMax || rate == bb::kN8) return 0;
+    // at rate 65536 a single polarisation's spectra are transformed in pairs, the odd one beside an empty one
+    if (rate == 65536 && P == 1 && T % (2 * rate) != 0) T += rate;
     return A * F * T * P * sizeof(float2);
 }
 
@@ -970,22 +932,23 @@ extern "C" int blade_channelize(const void* in, void* out, void* workspace, uint
     if (!make_plan(N1, p1) || !make_plan(N2, p2))
         return set_error(BLADE_ERROR, "blade_channelize: rate %llu has a prime factor above 61", (unsigned long long)rate);
     float2* ws = static_cast<float2*>(workspace);
-    if (N1 == 256 && N2 == 256 && S * P <= 32) {
-        const uint64_t batches = A * F * S;
-        const size_t sm1 = (16 * P * kLd + 512) * sizeof(float2), sm2 = (32 * kLd + 256) * sizeof(float2);
-        const uint64_t cap = (uint64_t)sm_count() * 2;
-        const uint64_t g1 = batches * 16, g2 = A * F * 256;
+    if (N1 == 256 && N2 == 256 && S * P <= 32 && aligned16(workspace)) {
+        const uint32_t S32 = (uint32_t)S, Su = P == 2 ? S32 : (S32 + 1) / 2, kk = rows_kk(Su);
+        const uint64_t rows = A * F, cap = (uint64_t)sm_count() * 2, g1 = rows * Su * 16, g2 = rows * (256 / kk);
+        const unsigned n1 = (unsigned)(g1 < cap ? g1 : cap), n2 = (unsigned)(g2 < cap ? g2 : cap);
+        const size_t sm2 = rows_smem(kk);
+        float4* w4 = static_cast<float4*>(workspace);
         int rc;
         if (P == 2) {
-            if ((rc = prepare_smem(fft256_cols_kernel<2>, sm1))) return rc;
-            if ((rc = prepare_smem(fft256_rows_kernel<2>, sm2))) return rc;
-            fft256_cols_kernel<2><<<(unsigned)(g1 < cap ? g1 : cap), 512, sm1, s>>>(in, ws, batches);
-            fft256_rows_kernel<2><<<(unsigned)(g2 < cap ? g2 : cap), 512, sm2, s>>>(ws, dst, A * F, (uint32_t)S);
+            if ((rc = prepare_smem(fft256_cols_kernel<2, false>, k65ColsSmem))) return rc;
+            if ((rc = prepare_smem(fft256_rows_kernel<2, 0, float>, sm2))) return rc;
+            fft256_cols_kernel<2, false><<<n1, k65Threads, k65ColsSmem, s>>>(in, w4, rows, S32);
+            fft256_rows_kernel<2, 0, float><<<n2, k65Threads, sm2, s>>>(w4, out, rows, S32, kk, 1, 0);
         } else {
-            if ((rc = prepare_smem(fft256_cols_kernel<1>, sm1))) return rc;
-            if ((rc = prepare_smem(fft256_rows_kernel<1>, sm2))) return rc;
-            fft256_cols_kernel<1><<<(unsigned)(g1 < cap ? g1 : cap), 512, sm1, s>>>(in, ws, batches);
-            fft256_rows_kernel<1><<<(unsigned)(g2 < cap ? g2 : cap), 512, sm2, s>>>(ws, dst, A * F, (uint32_t)S);
+            if ((rc = prepare_smem(fft256_cols_kernel<1, false>, k65ColsSmem))) return rc;
+            if ((rc = prepare_smem(fft256_rows_kernel<1, 0, float>, sm2))) return rc;
+            fft256_cols_kernel<1, false><<<n1, k65Threads, k65ColsSmem, s>>>(in, w4, rows, S32);
+            fft256_rows_kernel<1, 0, float><<<n2, k65Threads, sm2, s>>>(w4, out, rows, S32, kk, 1, 0);
         }
         return check_launch("blade_channelize");
     }
@@ -1124,27 +1087,26 @@ int spectrometer_launch(int in_type, const void* in, int out_type, void* out, vo
                         uint64_t T, uint64_t integration, uint64_t out_pols, int circular,
                         const uint32_t (&per_sm)[2], cudaStream_t s) {
     const uint64_t S = T / 65536;
-    float2* ws = static_cast<float2*>(workspace);
-    const uint64_t batches = A * F * S;
-    const size_t sm1 = (16 * 2 * kLd + 512) * sizeof(float2), sm2 = (32 * kLd + 256) * sizeof(float2);
+    float4* ws = static_cast<float4*>(workspace);
+    const uint32_t S32 = (uint32_t)S, I32 = (uint32_t)integration, kk = rows_kk(S32);
+    const uint64_t rows = A * F, g1 = rows * S * 16, g2 = rows * (256 / kk);
     const uint64_t cap1 = (uint64_t)sm_count() * per_sm[0], cap2 = (uint64_t)sm_count() * per_sm[1];
-    const uint64_t g1 = batches * 16, g2 = A * F * 256;
     const unsigned grid1 = (unsigned)(g1 < cap1 ? g1 : cap1), grid2 = (unsigned)(g2 < cap2 ? g2 : cap2);
+    const size_t sm2 = rows_smem(kk);
     int rc;
     if (in_type == BLADE_CI8) {
-        if ((rc = prepare_smem(fft256_cols_kernel<2, true>, sm1))) return rc;
-        fft256_cols_kernel<2, true><<<grid1, 512, sm1, s>>>(in, ws, batches);
+        if ((rc = prepare_smem(fft256_cols_kernel<2, true>, k65ColsSmem))) return rc;
+        fft256_cols_kernel<2, true><<<grid1, k65Threads, k65ColsSmem, s>>>(in, ws, rows, S32);
     } else {
-        if ((rc = prepare_smem(fft256_cols_kernel<2, false>, sm1))) return rc;
-        fft256_cols_kernel<2, false><<<grid1, 512, sm1, s>>>(in, ws, batches);
+        if ((rc = prepare_smem(fft256_cols_kernel<2, false>, k65ColsSmem))) return rc;
+        fft256_cols_kernel<2, false><<<grid1, k65Threads, k65ColsSmem, s>>>(in, ws, rows, S32);
     }
     if ((rc = check_launch("blade_spectrometer"))) return rc;
-    const uint32_t S32 = (uint32_t)S, I32 = (uint32_t)integration;
-#define BB_SPEC_ROWS(OPN, OTY)                                                                              \
-    do {                                                                                                    \
-        if ((rc = prepare_smem(fft256_rows_detect_kernel<OPN, OTY>, sm2))) return rc;                       \
-        fft256_rows_detect_kernel<OPN, OTY><<<grid2, 512, sm2, s>>>(ws, static_cast<OTY*>(out), A * F, S32, \
-                                                                    I32, circular ? 1 : 0);                 \
+#define BB_SPEC_ROWS(OPN, OTY)                                                                               \
+    do {                                                                                                     \
+        if ((rc = prepare_smem(fft256_rows_kernel<2, OPN, OTY>, sm2))) return rc;                            \
+        fft256_rows_kernel<2, OPN, OTY><<<grid2, k65Threads, sm2, s>>>(ws, out, rows, S32, kk, I32,          \
+                                                                       circular ? 1 : 0);                    \
     } while (0)
     if (out_type == BLADE_F32) {
         if (out_pols == 1) BB_SPEC_ROWS(1, float);
