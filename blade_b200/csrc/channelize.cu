@@ -558,6 +558,87 @@ __global__ void __launch_bounds__(256, 2) fft8192_kernel(const float2* __restric
     }
 }
 
+// The same transform for long two-polarisation blocks: a unit is both polarisations
+// of a spectrum as pairs (fft_regs.cuh), so that loads and stores move whole 16-byte
+// samples (one polarisation of a sample is 8 bytes of every 16 in, and of every 16 S
+// out) and the arithmetic is packed.  512 threads hold the 128 KB unit as 16 pairs
+// each, one CTA per SM; rows padded as above.  A row k1 belongs to one warp in stage
+// B, which rewrites it in place; in stage C two lanes share a 32-point DFT, one the
+// DFT-16 of its even samples, the other that of its odd ones, and swap their results
+// with lane shuffles.  Every value is rounded as in the kernel above.
+//
+// 8 x 192 rows of two spectra: 222 us against 324 us above; 16 x 192 rows of one: 176
+// against 206.  The stages of the one unit do not overlap (FP32 pipe about 3 us,
+// shared memory 3 us of 8.7 us per unit); asynchronous copies of the next unit into
+// shared memory during the stores change nothing (235 us).
+constexpr uint32_t kPairThreads8 = 512;
+
+__global__ void __launch_bounds__(kPairThreads8, 1) fft8192_pair_kernel(const float4* __restrict__ in,
+                                                                        float4* __restrict__ out, uint64_t units,
+                                                                        uint32_t S) {
+    extern __shared__ __align__(16) float4 ex[];  // 16 rows of kZ1
+    const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+    auto put = [&](uint32_t i, const fft::c2& v) { ex[i] = make_float4(v.re.x, v.re.y, v.im.x, v.im.y); };
+    auto get = [&](uint32_t i) {
+        const float4 q = ex[i];
+        return fft::c2{make_float2(q.x, q.y), make_float2(q.z, q.w)};
+    };
+    float2 wa, wb;
+    sincospif(-2.f * (float)tid / 8192.f, &wa.y, &wa.x);  // w8192^t, t = tid
+    sincospif(-2.f * (float)lane / 512.f, &wb.y, &wb.x);  // w512^v, v = lane
+    for (uint64_t unit = blockIdx.x; unit < units; unit += gridDim.x) {
+        fft::c2 v[16];
+        const float4* src = in + unit * kN8 + tid;
+#pragma unroll
+        for (int m = 0; m < 16; m++) v[m] = fft::pair(src[512 * m]);
+        if (tid < 32 && unit + gridDim.x < units)  // the next unit into L2 while this one runs
+            tc::prefetch_l2_bulk(in + (unit + gridDim.x) * kN8 + 256 * tid, 4096u);
+        fft::dft<16>(v);
+        float2 wk = make_float2(1.f, 0.f);
+        put(tid, v[0]);
+#pragma unroll
+        for (int k = 1; k < 16; k++) {
+            wk = cmul(wk, wa);
+            put(k * kZ1 + tid, fft::mul(v[k], wk));
+        }
+        __syncthreads();
+        {
+            const uint32_t row = warp * kZ1 + lane;  // k1 = warp, v = lane
+#pragma unroll
+            for (int u = 0; u < 16; u++) v[u] = get(row + 32 * u);
+            fft::dft<16>(v);
+            wk = make_float2(1.f, 0.f);
+            __syncwarp();
+            put(row, v[0]);
+#pragma unroll
+            for (int k = 1; k < 16; k++) {
+                wk = cmul(wk, wb);
+                put(row + k * kZ2, fft::mul(v[k], wk));
+            }
+        }
+        __syncthreads();
+        const uint32_t k1 = lane & 15u, h = lane >> 4, k2a = warp;
+#pragma unroll
+        for (int i = 0; i < 16; i++) v[i] = get(k1 * kZ1 + k2a * kZ2 + 2 * i + h);
+        __syncthreads();  // the next unit may overwrite the rows
+        fft::dft<16>(v);
+        const uint64_t af = unit / S;
+        float4* dst = out + af * kN8 * S + (uint32_t)(unit - af * S);
+        const float2 sign = fft::dup(h ? -1.f : 1.f);
+#pragma unroll
+        for (int k = 0; k < 16; k++) {
+            // X[k0] = e + w32^k o in the even lane, X[k0 + 4096] = e - w32^k o in the odd one
+            fft::c2 x = v[k];
+            if (h) x = fft::mul(x, c_w32[k]);
+            const fft::c2 y{make_float2(__shfl_xor_sync(0xffffffffu, x.re.x, 16), __shfl_xor_sync(0xffffffffu, x.re.y, 16)),
+                            make_float2(__shfl_xor_sync(0xffffffffu, x.im.x, 16), __shfl_xor_sync(0xffffffffu, x.im.y, 16))};
+            const fft::c2 r{__ffma2_rn(x.re, sign, y.re), __ffma2_rn(x.im, sign, y.im)};
+            const uint32_t k0 = k1 + 16 * k2a + 256 * k + 4096 * h;
+            dst[(uint64_t)((k0 + 4096u) & 8191u) * S] = fft::unpair(r, 0);
+        }
+    }
+}
+
 // ---- rate 65536 = 256 x 256 on pairs of transforms (fft_regs.cuh) ------------
 // n = j2 + 256 j1, k = k1 + 256 k2:
 //   W[k1][j2] = sum_j1 x[j2 + 256 j1] w256^(j1 k1)                    (column step)
@@ -906,6 +987,16 @@ extern "C" int blade_channelize(const void* in, void* out, void* workspace, uint
     const uint64_t S = T / rate;
     const int blocks_per_sm = 2;
     if (rate <= kSmallMax) return channelize_small("blade_channelize", src, false, dst, A, F, T, P, rate, 0, s);
+    if (rate == kN8 && P == 2 && A * F * S >= (S == 1 ? 8ull : 2ull) * sm_count()) {
+        // With one spectrum per row an 8-byte unit wastes half of each store, with more
+        // three quarters and beyond: pairs pay from eight spectra per SM (900 spectra 69
+        // against 67 us, 450 37 against 44) or from two (300 spectra 36 against 33 us).
+        const size_t smem = 16 * kZ1 * sizeof(float4);
+        if (int rc = prepare_smem(fft8192_pair_kernel, smem)) return rc;
+        fft8192_pair_kernel<<<(unsigned)sm_count(), kPairThreads8, smem, s>>>(
+            static_cast<const float4*>(in), static_cast<float4*>(out), A * F * S, (uint32_t)S);
+        return check_launch("blade_channelize");
+    }
     if (rate == kN8) {
         const uint64_t units = A * F * S * P;
         const size_t smem = 16 * kZ1 * sizeof(float2);

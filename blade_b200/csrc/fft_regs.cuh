@@ -25,9 +25,10 @@ __device__ __forceinline__ c2 sub(const c2& a, const c2& b) { return {sub2(a.re,
 __device__ __forceinline__ c2 add_mi(const c2& a, const c2& b) { return {__fadd2_rn(a.re, b.im), sub2(a.im, b.re)}; }
 __device__ __forceinline__ c2 sub_mi(const c2& a, const c2& b) { return {sub2(a.re, b.im), __fadd2_rn(a.im, b.re)}; }
 __device__ __forceinline__ float2 dup(float v) { return make_float2(v, v); }
-// a * w for one twiddle w shared by the pair
+// a * w for one twiddle w shared by the pair: each member rounds as
+// (fma(a.re, w.re, -(a.im w.im)), fma(a.re, w.im, a.im w.re))
 __device__ __forceinline__ c2 mul(const c2& a, float wr, float wi) {
-    return {__ffma2_rn(a.im, dup(-wi), __fmul2_rn(a.re, dup(wr))), __ffma2_rn(a.im, dup(wr), __fmul2_rn(a.re, dup(wi)))};
+    return {__ffma2_rn(a.re, dup(wr), __fmul2_rn(a.im, dup(-wi))), __ffma2_rn(a.re, dup(wi), __fmul2_rn(a.im, dup(wr)))};
 }
 __device__ __forceinline__ c2 mul(const c2& a, float2 w) { return mul(a, w.x, w.y); }
 
