@@ -90,6 +90,7 @@ struct TcArgs {
     uint64_t total_tiles;
     uint32_t pdl;  // launched as a programmatic dependent of the phasor split: wait for it before the image
     uint32_t direct;  // R = 1 CI8 without a raw ring: converter threads load the voltages themselves
+    uint32_t circ;  // PRE: (X, Y) -> (X + iY, X - iY) while the operand is built
     uint32_t transposed;  // outputs along TMEM lanes, samples along columns (64-beam chunks, rate 1, I = 8 or 16)
 };
 
@@ -277,8 +278,20 @@ __device__ __forceinline__ R4Task r4_task(uint32_t wt, uint32_t lane, uint32_t A
     return t;
 }
 
+// Circular basis of one value of both polarisations, halves = (pol 0, pol 1):
+// (X + iY, X - iY), integers of magnitude <= 1024 here, exact in FP16.
+__device__ __forceinline__ void circular_h2(half2& re, half2& im) {
+    const half2 mp = __halves2half2(__float2half(-1.f), __float2half(1.f));
+    const half2 pm = __halves2half2(__float2half(1.f), __float2half(-1.f));
+    const half2 xr = __low2half2(re), yr = __high2half2(re), xi = __low2half2(im), yi = __high2half2(im);
+    re = __hfma2(yi, mp, xr);
+    im = __hfma2(yr, pm, xi);
+}
+
+// PRE = true: with g.circ the polarisations are rotated after the transform.
+template <bool PRE>
 __device__ __forceinline__ void r4_pair_task(const uint8_t* raw, uint32_t rrow, uint8_t* op0, uint8_t* op1,
-                                             const R4Task& t) {
+                                             const R4Task& t, uint32_t circ) {
     const half2 h2304 = __halves2half2(__ushort_as_half(0x6880), __ushort_as_half(0x6880));  // 2304
     uint2 out_r[2][4], out_i[2][4];  // [pol][k]
     if (t.nvalid) {
@@ -308,6 +321,10 @@ __device__ __forceinline__ void r4_pair_task(const uint8_t* raw, uint32_t rrow, 
             zi[i][2] = __hadd2(aI, bI);
             zr[i][3] = __hadd2(cR, dI);  // x0 - i x1 - x2 + i x3
             zi[i][3] = __hsub2(cI, dR);
+            if (PRE && circ) {
+#pragma unroll
+                for (int k = 0; k < 4; k++) circular_h2(zr[i][k], zi[i][k]);
+            }
         }
 #pragma unroll
         for (int p = 0; p < 2; p++) {
@@ -332,6 +349,64 @@ __device__ __forceinline__ void r4_pair_task(const uint8_t* raw, uint32_t rrow, 
         *reinterpret_cast<uint2*>(op0 + t.o_i + k * 4096u) = out_i[0][k];
         *reinterpret_cast<uint2*>(op1 + t.o_r + k * 4096u) = out_r[1][k];
         *reinterpret_cast<uint2*>(op1 + t.o_i + k * 4096u) = out_i[1][k];
+    }
+}
+
+// R = 2, both polarisations in one pass, arranged as the R = 4 tasks above: a warp
+// covers 16 of the tile's 64 spectra x 8 antennas, row k * 64 + s sits 8192 * k bytes
+// after row s, and the DFT runs on (p0, p1) halves (x0 - x1: the 1152 biases cancel;
+// x0 + x1: removed together).
+__device__ __forceinline__ R4Task r2_task(uint32_t wt, uint32_t lane, uint32_t A, uint32_t KA, uint32_t rrow) {
+    const uint32_t s = (wt & 3u) * 16u + (lane & 7u) + ((lane >> 4) << 3);
+    const uint32_t a0 = (2u * (wt >> 2) + ((lane >> 3) & 1u)) * 4u;
+    R4Task t;
+    t.raw_off = a0 * rrow + s * 8u;
+    t.o_r = op_off(s, a0);
+    t.o_i = op_off(s, KA + a0);
+    t.nvalid = a0 < A ? min(4u, A - a0) : 0u;
+    return t;
+}
+
+template <bool PRE>
+__device__ __forceinline__ void r2_pair_task(const uint8_t* raw, uint32_t rrow, uint8_t* op0, uint8_t* op1,
+                                             const R4Task& t, uint32_t circ) {
+    const half2 h2304 = __halves2half2(__ushort_as_half(0x6880), __ushort_as_half(0x6880));  // 2304
+    half2 zr[4][2], zi[4][2];  // [antenna][k], halves = (pol 0, pol 1)
+#pragma unroll
+    for (uint32_t i = 0; i < 4; i++) {
+        if (i < t.nvalid) {
+            const uint2 v = *reinterpret_cast<const uint2*>(raw + t.raw_off + i * rrow);
+            const uint32_t w[2] = {v.x ^ 0x80808080u, v.y ^ 0x80808080u};
+            half2 re[2], im[2];  // 1152 + x
+#pragma unroll
+            for (int j = 0; j < 2; j++) {
+                re[j] = u2h(__byte_perm(w[j], 0x64646464u, 0x4240));
+                im[j] = u2h(__byte_perm(w[j], 0x64646464u, 0x4341));
+            }
+            zr[i][0] = __hsub2(re[0], re[1]);
+            zi[i][0] = __hsub2(im[0], im[1]);
+            zr[i][1] = __hadd2(__hsub2(re[0], h2304), re[1]);
+            zi[i][1] = __hadd2(__hsub2(im[0], h2304), im[1]);
+            if (PRE && circ) {
+#pragma unroll
+                for (int k = 0; k < 2; k++) circular_h2(zr[i][k], zi[i][k]);
+            }
+        } else {
+#pragma unroll
+            for (int k = 0; k < 2; k++) zr[i][k] = zi[i][k] = u2h(0u);
+        }
+    }
+#pragma unroll
+    for (int p = 0; p < 2; p++) {
+        const uint32_t sel = p ? 0x7632u : 0x5410u;
+        uint8_t* op = p ? op1 : op0;
+#pragma unroll
+        for (uint32_t k = 0; k < 2; k++) {
+            *reinterpret_cast<uint2*>(op + t.o_r + k * 8192u) =
+                make_uint2(__byte_perm(h2u(zr[0][k]), h2u(zr[1][k]), sel), __byte_perm(h2u(zr[2][k]), h2u(zr[3][k]), sel));
+            *reinterpret_cast<uint2*>(op + t.o_i + k * 8192u) =
+                make_uint2(__byte_perm(h2u(zi[0][k]), h2u(zi[1][k]), sel), __byte_perm(h2u(zi[2][k]), h2u(zi[3][k]), sel));
+        }
     }
 }
 
@@ -525,14 +600,6 @@ __device__ __forceinline__ void direct_build(const uint32_t (&v)[kDirectMaxJ][8]
 #pragma unroll
     for (uint32_t j = 0; j < kDirectMaxJ; j++)
         if (j < t.nj) r1_convert_store(v[j], op0, op1, t.o_r[j], t.o_i[j]);
-}
-
-// Both polarisations of one tile for R = 1 and 2: two single-polarisation passes.
-template <int R>
-__device__ __forceinline__ void build_operand_pair(const uint8_t* raw, uint32_t rrow, uint8_t* op0, uint8_t* op1, uint32_t A,
-                                                   uint32_t KA, uint32_t ct) {
-    build_operand<R>(raw, rrow, op0, A, KA, 0, ct);
-    build_operand<R>(raw, rrow, op1, A, KA, 1, ct);
 }
 
 // Window sum of NV per-beam values over I = 2^LOGI adjacent lanes by a butterfly
@@ -744,7 +811,19 @@ __device__ __forceinline__ void epilogue_transposed(const TcArgs& g, uint32_t tm
 }
 
 // ES = bytes per dual-polarisation input sample: 4 (CI8) or 8 (CF16, rate 1 only).
-template <int R, int LOGI, int ES = 4>
+//
+// PRE (ModeB's order, R = 2 or 4): the channelizer runs before the beamformer, so every
+// fine channel has its own phasors.  The operand is the same (row = k * 128 / R +
+// spectrum holds fine channel k), and the R fine channels' stacked images lie side
+// by side along N: one MMA of N = 4 R NB columns per k-step gives every row the
+// products of all R images, of which the epilogue reads the columns of the row's own
+// fine channel.  The tensor pipe does R times the useful work and is still not what
+// bounds the tile (1024 of about 1900 cycles at R = 4, NB = 16), and the fine-channel
+// voltages never reach memory (28 antennas x 192 channels x 8192 samples, 16 beams,
+// R = 4, I = 4: 96 us with the split, where CF16 fine channels through memory took 88
+// to write and 104 to beamform).  An accumulator is one polarisation (2 x 256 columns
+// fill tensor memory), and each MMA issuer owns one.
+template <int R, int LOGI, int ES = 4, bool PRE = false>
 __global__ void __launch_bounds__(kThreads, 1) bf_tc_kernel(const TcArgs g, const __grid_constant__ CUtensorMap tmap) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     // Swizzled operands need 1024-byte aligned atoms: align the working base.
@@ -772,11 +851,12 @@ __global__ void __launch_bounds__(kThreads, 1) bf_tc_kernel(const TcArgs g, cons
     volatile int never = 0;  // abort flag that is never raised (drain waits)
     // Accumulator columns per polarisation: [re | im] (2 NB), or with hi/lo stacked
     // along N [hi re | hi im | lo re | lo im] (4 NB).
-    const uint32_t d_cols = (g.stacked ? 4u : 2u) * NB;
+    const uint32_t d_cols = (PRE ? 4u * R : g.stacked ? 4u : 2u) * NB;
     // Accumulator buffers (tiles in flight between MMA and epilogue): as many as
     // fit the 512 TMEM columns, at most kMaxAcc.
-    const uint32_t nacc = min((uint32_t)kMaxAcc, 512u / (2u * d_cols));
-    const uint32_t need_cols = nacc * 2u * d_cols;
+    // PRE: one accumulator per polarisation.
+    const uint32_t nacc = PRE ? 2u : min((uint32_t)kMaxAcc, 512u / (2u * d_cols));
+    const uint32_t need_cols = (PRE ? 2u : nacc * 2u) * d_cols;
     const uint32_t tmem_cols = need_cols <= 32 ? 32 : need_cols <= 64 ? 64 : need_cols <= 128 ? 128 : need_cols <= 256 ? 256 : 512;
     // Pair mode: the converter builds both polarisations of a tile in one pass and
     // signals them together on the second stage of the pair.
@@ -787,17 +867,17 @@ __global__ void __launch_bounds__(kThreads, 1) bf_tc_kernel(const TcArgs g, cons
     // count is even, so that every barrier is only ever used by one issuer.  An
     // issue of tcgen05.mma holds its thread for about the MMA's duration, so one
     // issuer's waits and commits overlap the other's MMAs.
-    const uint32_t nis = (pair && ((AS / 2) & 1u) == 0 && (nacc & 1u) == 0) ? 2u : 1u;
+    const uint32_t nis = PRE || (pair && ((AS / 2) & 1u) == 0 && (nacc & 1u) == 0) ? 2u : 1u;
     // Split operand build (R = 4, two issuers, two-tile raw stages): converter warps
     // 0-3 build the even tiles of the CTA's range (the first tile of each raw stage,
     // issuer 0's) and warps 4-7 the odd ones, so the two halves run independently
     // and each operand pair has four producers.
-    const bool split = R == 4 && nis == 2 && g.raw_tiles == 2;
+    const bool split = R == 4 && nis == 2 && g.raw_tiles == 2;  // PRE: nis is always 2
 
     if (threadIdx.x == 0) {
         for (uint32_t i = 0; i < AS; i++) {
             mbar_init(&a_full[i], split ? kConvWarps / 2 : kConvWarps);
-            mbar_init(&a_empty[i], 1);
+            mbar_init(&a_empty[i], PRE ? 2 : 1);  // PRE: both issuers read the tile's pair
         }
         for (uint32_t i = 0; i < RS; i++) {
             mbar_init(&r_full[i], 1);
@@ -855,7 +935,7 @@ __global__ void __launch_bounds__(kThreads, 1) bf_tc_kernel(const TcArgs g, cons
             const uint32_t wpol16 = g.stacked ? (2 * KA / 64) * 4 * nb16 : (KA == 64 ? 6 * nb16 : 4 * nb16);
             // This issuer's first tile is local tile j: operand stage 2 j (pair mode)
             // or 0, accumulator j; both advance by nis tiles per own tile.
-            uint32_t as = pair ? 2 * j : 0, aph = 0, db = j, dph = 0, wph = 0;
+            uint32_t as = pair && !PRE ? 2 * j : 0, aph = 0, db = j, dph = 0, wph = 0;
             uint32_t tt = (uint32_t)(L0 % tpc);  // time tile within the channel, stepped below
             bool ok = true;
             uint32_t i = 0;
@@ -863,7 +943,22 @@ __global__ void __launch_bounds__(kThreads, 1) bf_tc_kernel(const TcArgs g, cons
                 if (L == L0 || tt == 0) {
                     if (!wait_all(w_full, wph, 1)) { ok = false; break; }
                 }
-                if ((i % nis) == j) {
+                if constexpr (PRE) {
+                    // issuer j: polarisation j of every tile into accumulator j
+                    if (!wait_all(&d_empty[j], dph ^ 1, 3) || !wait_all(&a_full[as + 1], aph, 2)) { ok = false; break; }
+                    tc_fence_after();
+                    if (lane == 0) {
+                        const uint64_t ad = a_desc + (uint64_t)((as + j) * op16), wd = w_desc + (uint64_t)(j * R * wpol16);
+                        if (KA == 64) issue_stacked<8>(tmem + j * d_cols, ad, wd, 4 * R * nb16, idesc);
+                        else issue_stacked<4>(tmem + j * d_cols, ad, wd, 4 * R * nb16, idesc);
+                        mma_commit(&a_empty[as + 1]);
+                        mma_commit(&d_full[j]);
+                    }
+                    __syncwarp();
+                    dph ^= 1;
+                    as += 2;
+                    if (as == AS) { as = 0; aph ^= 1; }
+                } else if ((i % nis) == j) {
                     if (!wait_all(&d_empty[db], dph ^ 1, 3)) { ok = false; break; }
                     const uint32_t np = pair ? 1u : 2u;  // operand handshakes per tile
                     for (uint32_t h = 0; h < np; h++) {
@@ -1011,6 +1106,66 @@ __global__ void __launch_bounds__(kThreads, 1) bf_tc_kernel(const TcArgs g, cons
                 done = true;
             }
         }
+        if constexpr (PRE) {
+            // ---------------- epilogue, one polarisation at a time ----------------
+            static_assert(kEpiGroups == 1, "one warp per lane quarter");
+            constexpr uint32_t I = 1u << LOGI, rows_per_k = kM / R;
+            constexpr int kB16 = R == 4 ? 1 : 2;  // 16-beam chunks at most (4 R NB <= 256 columns)
+            const uint32_t q = warp & 3, row = 32 * q + lane, k = row / rows_per_k, s_local = row - k * rows_per_k;
+            const uint64_t bstride = (uint64_t)g.F * R * g.U;
+            uint32_t dph = 0, f = (uint32_t)(L0 / tpc), tt = (uint32_t)(L0 % tpc);
+            bool ok = true;
+            for (uint64_t L = L0; L < L1 && ok; L++) {
+                float2 pw2[kB16][8];
+#pragma unroll
+                for (int c = 0; c < kB16; c++)
+#pragma unroll
+                    for (int j = 0; j < 8; j++) pw2[c][j] = make_float2(0.f, 0.f);
+                for (uint32_t p = 0; p < 2; p++) {
+                    if (!mbar_wait(&d_full[p], dph, abort, kWaitBudget)) { record_abort(abort, 7); ok = false; break; }
+                    tc_fence_after();
+                    const uint32_t pa = tmem + ((32 * q) << 16) + p * d_cols + k * 4 * NB;
+#pragma unroll
+                    for (int c = 0; c < kB16; c++) {
+                        if (16u * c >= NB) break;
+                        uint32_t hr[16], hi[16], lr[16], li[16];
+                        tmem_ld(pa + 16 * c, hr);
+                        tmem_ld(pa + NB + 16 * c, hi);
+                        tmem_ld(pa + 2 * NB + 16 * c, lr);
+                        tmem_ld(pa + 3 * NB + 16 * c, li);
+                        tmem_ld_wait();
+#pragma unroll
+                        for (int j = 0; j < 8; j++) {
+                            const float2 a = __fadd2_rn(make_float2(__uint_as_float(hr[2 * j]), __uint_as_float(hr[2 * j + 1])),
+                                                        make_float2(__uint_as_float(lr[2 * j]), __uint_as_float(lr[2 * j + 1])));
+                            const float2 b = __fadd2_rn(make_float2(__uint_as_float(hi[2 * j]), __uint_as_float(hi[2 * j + 1])),
+                                                        make_float2(__uint_as_float(li[2 * j]), __uint_as_float(li[2 * j + 1])));
+                            pw2[c][j] = __ffma2_rn(a, a, __ffma2_rn(b, b, pw2[c][j]));
+                        }
+                    }
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&d_empty[p]);
+                }
+                if (!ok) break;
+                float* obase = g.out + ((uint64_t)f * R + k) * g.U + (tt * rows_per_k + s_local) / I;
+#pragma unroll
+                for (int c = 0; c < kB16; c++) {
+                    if (16u * c >= NB) break;
+                    uint32_t first;
+                    float(&pw)[16] = *reinterpret_cast<float(*)[16]>(pw2[c]);
+                    const int cnt = window_reduce<16, LOGI>(pw, lane, &first);
+#pragma unroll
+                    for (int j = 0; j < 16; j++) {
+                        const uint32_t b = 16 * c + first + j;
+                        if (j < cnt && b < g.beams) obase[b * bstride] = pw[j];
+                    }
+                }
+                dph ^= 1;
+                if (++tt == tpc) { tt = 0; f++; }
+            }
+            done = true;
+        }
         if (!done) {
             // ---------------- epilogue ----------------
             constexpr uint32_t I = 1u << LOGI;
@@ -1116,7 +1271,7 @@ __global__ void __launch_bounds__(kThreads, 1) bf_tc_kernel(const TcArgs g, cons
                     uint8_t* op1 = op0 + op_bytes;
 #pragma unroll
                     for (uint32_t i = 0; i < kMaxTk; i++)
-                        if (i < ntk) r4_pair_task(raw, g.raw_row, op0, op1, tk[i]);
+                        if (i < ntk) r4_pair_task<PRE>(raw, g.raw_row, op0, op1, tk[i], g.circ);
                     fence_proxy_async_smem();
                     __syncwarp();
                     if (lane == 0) {
@@ -1183,6 +1338,14 @@ __global__ void __launch_bounds__(kThreads, 1) bf_tc_kernel(const TcArgs g, cons
 #pragma unroll
             for (uint32_t i = 0; i < kMaxT4; i++) t4[i] = r4_task((ct >> 5) + i * kConvWarps, lane, g.A, KA, g.raw_row);
         }
+        // R = 2 pair mode: KA / 2 warp-tasks
+        constexpr uint32_t kMaxT2 = kMaxKA / 2 / kConvWarps;
+        const uint32_t nt2 = KA / 2 / kConvWarps;
+        R4Task t2[kMaxT2];
+        if constexpr (R == 2) {
+#pragma unroll
+            for (uint32_t i = 0; i < kMaxT2; i++) t2[i] = r2_task((ct >> 5) + i * kConvWarps, lane, g.A, KA, g.raw_row);
+        }
         R1Task t1;
         if constexpr (R == 1 && ES == 4) t1 = r1_task(ct >> 5, lane, g.A, KA, g.raw_row);
         uint32_t rs = 0, rph = 0, as = 0, aph = 0;
@@ -1206,13 +1369,15 @@ __global__ void __launch_bounds__(kThreads, 1) bf_tc_kernel(const TcArgs g, cons
                 if constexpr (R == 4) {
 #pragma unroll
                     for (uint32_t i = 0; i < kMaxT4; i++)
-                        if (i < nt4) r4_pair_task(raw, g.raw_row, op0, op1, t4[i]);
+                        if (i < nt4) r4_pair_task<PRE>(raw, g.raw_row, op0, op1, t4[i], g.circ);
                 } else if constexpr (ES == 8) {
                     build_operand_h16_pair(raw, g.raw_row, op0, op1, g.A, KA, ct);
                 } else if constexpr (R == 1) {
                     r1_pair_task(raw, g.raw_row, op0, op1, t1);
                 } else {
-                    build_operand_pair<R>(raw, g.raw_row, op0, op1, g.A, KA, ct);
+#pragma unroll
+                    for (uint32_t i = 0; i < kMaxT2; i++)
+                        if (i < nt2) r2_pair_task<PRE>(raw, g.raw_row, op0, op1, t2[i], g.circ);
                 }
                 fence_proxy_async_smem();
                 __syncwarp();
@@ -1278,7 +1443,7 @@ __device__ __forceinline__ void put_chunk(uint8_t* base, uint32_t rows, uint32_t
 __global__ void __launch_bounds__(256) tc_prepare_kernel(const float2* __restrict__ ph, uint8_t* __restrict__ plan,
                                                          uint32_t B, uint32_t A, uint32_t F, uint32_t NB,
                                                          uint32_t KA, uint32_t nchunks, uint32_t img_bytes,
-                                                         uint32_t stacked) {
+                                                         uint32_t stacked, uint32_t fold) {
     // a chain kernel launched as this grid's programmatic dependent may start its
     // prologue now; it waits for this grid to finish before it reads the image
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -1319,16 +1484,17 @@ __global__ void __launch_bounds__(256) tc_prepare_kernel(const float2* __restric
         if (stacked) {
             // per p, (2 KA / 64) column blocks of 4 NB rows:
             //   hi: row nb -> [Wr | -Wi], row NB + nb -> [Wi | Wr]; lo: the same at rows + 2 NB
-            uint8_t* base = plan + ((uint64_t)c * F + f) * img_bytes + (uint64_t)p * pol_stacked;
-            const uint32_t rows = 4 * NB;
-            put_chunk(base, rows, nb, k0, pack8(rh));
-            put_chunk(base, rows, nb, KA + k0, pack8(nih));
-            put_chunk(base, rows, NB + nb, k0, pack8(ih));
-            put_chunk(base, rows, NB + nb, KA + k0, pack8(rh));
-            put_chunk(base, rows, 2 * NB + nb, k0, pack8(rl));
-            put_chunk(base, rows, 2 * NB + nb, KA + k0, pack8(nil));
-            put_chunk(base, rows, 3 * NB + nb, k0, pack8(il));
-            put_chunk(base, rows, 3 * NB + nb, KA + k0, pack8(rl));
+            // fold > 1: the images of fold consecutive channels as one, rows stacked per polarisation
+            const uint32_t fk = f % fold, r0 = fk * 4 * NB + nb, rows = fold * 4 * NB;
+            uint8_t* base = plan + ((uint64_t)c * F + (f - fk)) * img_bytes + (uint64_t)p * fold * pol_stacked;
+            put_chunk(base, rows, r0, k0, pack8(rh));
+            put_chunk(base, rows, r0, KA + k0, pack8(nih));
+            put_chunk(base, rows, r0 + NB, k0, pack8(ih));
+            put_chunk(base, rows, r0 + NB, KA + k0, pack8(rh));
+            put_chunk(base, rows, r0 + 2 * NB, k0, pack8(rl));
+            put_chunk(base, rows, r0 + 2 * NB, KA + k0, pack8(nil));
+            put_chunk(base, rows, r0 + 3 * NB, k0, pack8(il));
+            put_chunk(base, rows, r0 + 3 * NB, KA + k0, pack8(rl));
             continue;
         }
         uint8_t* base = plan + ((uint64_t)c * F + f) * img_bytes + (uint64_t)p * 2 * ph_bytes;
@@ -1663,7 +1829,7 @@ extern "C" int blade_beamform_tc_prepare(const void* phasors, void* plan, uint64
     } else {
         tc_prepare_kernel<<<grid_for(n, 256), 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
             static_cast<const float2*>(phasors), static_cast<uint8_t*>(plan), (uint32_t)B, (uint32_t)A, (uint32_t)F,
-            s.NB, s.KA, s.nchunks, s.img_bytes, s.stacked);
+            s.NB, s.KA, s.nchunks, s.img_bytes, s.stacked, 1u);
     }
     return check_launch("blade_beamform_tc_prepare");
 }
@@ -1721,6 +1887,7 @@ int tc_run(const char* who, const void* in, const void* plan, void* out, uint64_
         g.total_tiles = (uint64_t)F * (T / kM);
         g.pdl = (pdl && c == 0) ? 1u : 0u;
         g.direct = s.direct;
+        g.circ = 0;
         // outputs along TMEM lanes: full 64-beam chunks (separate hi/lo products),
         // rate 1 CI8, windows of 8 or 16 samples, 16-byte aligned output rows
         g.transposed = (!s.stacked && s.NB == 64 && rate == 1 && es == 4 && (integration == 8 || integration == 16) &&
@@ -1836,6 +2003,118 @@ extern "C" int blade_beamform_prepare_detect_tc_cf16(const void* phasors, void* 
     if (int rc = blade_beamform_tc_prepare(phasors, plan, B, A, F, P, stream)) return rc;
     return tc_run("blade_beamform_prepare_detect_tc_cf16", in, plan, out, B, A, F, T, 1, integration, 8,
                   pick_cf16(integration), stream, true);
+}
+
+namespace bb {
+namespace {
+
+// Layout of the PRE chain: up to 32 antennas, one chunk of beams whose R stacked images
+// fit an MMA's 256 columns; three operand tile pairs and two two-tile raw stages (one
+// KB rows) beside the 64 KB of images, or as many one-tile stages as fit when a
+// channel's tiles are odd.
+bool pre_shape(uint64_t B, uint64_t A, uint64_t T, uint64_t rate, TcShape& s) {
+    if (rate != 2 && rate != 4) return false;
+    if (!tc_shape(B, A, s) || s.KA != 32 || s.nchunks != 1 || !s.stacked || 4 * rate * s.NB > 256) return false;
+    const size_t op = (2ull * s.KA / 64) * 16384, limit = 227 * 1024;
+    s.direct = 0;
+    s.a_stages = 6;
+    s.raw_tiles = (T / kM) % 2 == 0 ? 2u : 1u;
+    s.raw_row = s.raw_tiles * kM * 4;
+    s.raw_bytes = (uint32_t)A * s.raw_row;
+    const size_t fixed = rate * (size_t)s.img_bytes + 1536 + s.a_stages * op;
+    s.r_stages = 2;
+    while (s.r_stages < 4 && fixed + (s.r_stages + 1) * (size_t)s.raw_bytes <= limit) s.r_stages++;
+    s.smem = fixed + s.r_stages * (size_t)s.raw_bytes;
+    return s.smem <= limit;
+}
+
+template <int R>
+TcKernel pick_pre(uint64_t integration) {
+    switch (integration) {
+        case 1: return bf_tc_kernel<R, 0, 4, true>;
+        case 2: return bf_tc_kernel<R, 1, 4, true>;
+        case 4: return bf_tc_kernel<R, 2, 4, true>;
+        case 8: return bf_tc_kernel<R, 3, 4, true>;
+        case 16: return bf_tc_kernel<R, 4, 4, true>;
+        default: return bf_tc_kernel<R, 5, 4, true>;
+    }
+}
+
+}  // namespace
+}  // namespace bb
+
+extern "C" int blade_modeb_detect_tc_supported(uint64_t B, uint64_t A, uint64_t F, uint64_t T, uint64_t P,
+                                               uint64_t rate, uint64_t integration) {
+    TcShape s;
+    if (rate == 1 || !blade_beamform_detect_tc_supported(B, A, F, T, P, rate, integration)) return 0;
+    // windows of rate x integration samples must tile a channel, and close inside a tile's rows
+    if (T % (rate * integration) != 0 || integration > kM / rate) return 0;
+    const uint64_t split = F * rate * 2 * 64 * 4;  // threads of the split at most
+    return split <= 0xFFFFFFFFull && pre_shape(B, A, T, rate, s) ? 1 : 0;
+}
+
+extern "C" int blade_modeb_detect_tc(const void* phasors, void* plan, const void* in, void* out, uint64_t B,
+                                     uint64_t A, uint64_t F, uint64_t T, uint64_t P, uint64_t rate,
+                                     uint64_t integration, int circular, blade_stream_t stream) {
+    const char* who = "blade_modeb_detect_tc";
+    if (!blade_modeb_detect_tc_supported(B, A, F, T, P, rate, integration))
+        return set_error(BLADE_ERROR,
+                         "%s: unsupported configuration (B=%llu A=%llu T=%llu P=%llu rate=%llu I=%llu): needs P=2, "
+                         "1<=A<=32, rate 4 with B<=16 or 2 with B<=32, T%%128==0, I a power of two <= 32", who,
+                         (unsigned long long)B, (unsigned long long)A, (unsigned long long)T, (unsigned long long)P,
+                         (unsigned long long)rate, (unsigned long long)integration);
+    if (!in || !plan || !out || !phasors) return set_error(BLADE_ERROR, "%s: null buffer", who);
+    if (!aligned16(in) || !aligned16(plan) || (reinterpret_cast<uintptr_t>(out) & 3))
+        return set_error(BLADE_ERROR, "%s: input and plan must be 16-byte aligned", who);
+    TcShape s;
+    pre_shape(B, A, T, rate, s);
+    cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+    const uint32_t FR = (uint32_t)(F * rate);
+    const uint64_t n = (uint64_t)FR * 2 * s.NB * (s.KA / 8);
+    tc_prepare_kernel<<<grid_for(n, 256), 256, 0, st>>>(static_cast<const float2*>(phasors),
+                                                      static_cast<uint8_t*>(plan), (uint32_t)B, (uint32_t)A, FR, s.NB,
+                                                      s.KA, 1u, s.img_bytes, 1u, (uint32_t)rate);
+    if (int rc = check_launch(who)) return rc;
+    const TcKernel fn = rate == 4 ? pick_pre<4>(integration) : pick_pre<2>(integration);
+    if (int rc = ensure_smem(reinterpret_cast<const void*>(fn), s.smem)) return rc;
+    CUtensorMap tmap;
+    if (int rc = encode_voltage_map(&tmap, in, A, F, T, s.raw_row / 4, 4)) return rc;
+    TcArgs g = {};
+    g.in = static_cast<const uint8_t*>(in);
+    g.plan = static_cast<const uint8_t*>(plan);
+    g.out = static_cast<float*>(out);
+    g.A = (uint32_t)A;
+    g.F = (uint32_t)F;
+    g.T = (uint32_t)T;
+    g.beams = (uint32_t)B;
+    g.U = (uint32_t)(T / (rate * integration));
+    g.NB = s.NB;
+    g.KA = s.KA;
+    g.a_stages = s.a_stages;
+    g.r_stages = s.r_stages;
+    g.stacked = 1;
+    g.img_bytes = (uint32_t)rate * s.img_bytes;
+    g.raw_bytes = s.raw_bytes;
+    g.raw_tiles = s.raw_tiles;
+    g.raw_row = s.raw_row;
+    g.tiles_per_ch = (uint32_t)(T / kM);
+    g.total_tiles = (uint64_t)F * g.tiles_per_ch;
+    g.pdl = 1;
+    g.circ = circular ? 1u : 0u;
+    const uint64_t sms = (uint64_t)sm_count();
+    const uint64_t per = ((g.total_tiles + sms - 1) / sms + s.raw_tiles - 1) / s.raw_tiles * s.raw_tiles;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)((g.total_tiles + per - 1) / per), 1, 1);
+    cfg.blockDim = dim3(kThreads, 1, 1);
+    cfg.dynamicSmemBytes = s.smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, fn, g, tmap);
+    return e != cudaSuccess ? check_cuda(e, who) : check_launch(who);
 }
 
 namespace bb {

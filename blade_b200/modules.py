@@ -869,12 +869,17 @@ class ModeH(Module):
 
 
 class _ModeBTensorCore(Module):
-    """ModeB on CI8 voltages with the detector (Stokes-I) at channelizer rate 2 or 4:
-    the pre-beamformer Cast -> Channelizer -> [Polarizer] into an exact CF16 buffer
-    (blade_prechannelize_cf16), then the per-fine-channel phasor split and the
-    tensor-core Beamformer -> Detector at rate 1 (blade_beamform_prepare_detect_tc_cf16:
-    the split, then the chain overlapping its end), and with the incoherent beam its detected row
-    (blade_incoherent_detect_cf16).  Three or four launches."""
+    """ModeB on CI8 voltages with the detector (Stokes-I) at channelizer rate 2 or 4,
+    on tensor cores with per-fine-channel phasors.
+
+    direct (blade_modeb_detect_tc: up to 32 antennas, 16 beams at rate 4 or 32 at
+    rate 2): the phasor split and one chain from the CI8 block, which transforms and
+    polarizes while it builds its operand; the detected incoherent beam, when
+    enabled, also comes from the CI8 block (blade_incoherent_detect_ci8).
+    Otherwise the pre-beamformer stages go to an exact CF16 buffer
+    (blade_prechannelize_cf16) that the split and chain
+    (blade_beamform_prepare_detect_tc_cf16) and the incoherent beam
+    (blade_incoherent_detect_cf16) read."""
 
     taint = Taint.CONSUMER | Taint.PRODUCER
 
@@ -885,10 +890,16 @@ class _ModeBTensorCore(Module):
         A, F, T, P = as_vector(buffer).shape
         B = as_vector(phasors).shape[0]
         R = self._R
-        self._pre = self._alloc((A, F * R, T // R, P), "cf16")
+        self.direct = self._direct(A, F, T, P, B, R, self._I)
+        self._pre = None if self.direct else self._alloc((A, F * R, T // R, P), "cf16")
         n = int(_lib.load().blade_beamform_tc_plan_size(B, A, F * R, P))
         self._plan = self._alloc((n,), "i8", "tensor")
         self._output = self._alloc((B + int(self._inc), F * R, T // (R * self._I), 1), "f32")
+
+    @staticmethod
+    def _direct(A, F, T, P, B, R, I) -> bool:
+        # the incoherent beam takes one grid row per coarse channel
+        return F <= 65535 and _lib.load().blade_modeb_detect_tc_supported(B, A, F, T, P, R, I) == 1
 
     @staticmethod
     def applies(it, A, F, T, P, B, R, I, detector, OP) -> bool:
@@ -901,14 +912,22 @@ class _ModeBTensorCore(Module):
 
     def process(self, step=0, stream=None):
         x, ph = as_vector(self._buffer), as_vector(self._phasors)
-        pre, plan, out = _out(self._pre), _out(self._plan), _out(self._output)
+        plan, out = _out(self._plan), _out(self._output)
         A, F, T, P = x.shape
         B, R, sh = ph.shape[0], self._R, _stream_handle(stream)
+        row = out.data_ptr() + B * F * R * (T // (R * self._I)) * 4  # beam row B: the incoherent beam
+        if self.direct:
+            _lib.call("blade_modeb_detect_tc", ph.data_ptr(), plan.data_ptr(), x.data_ptr(), out.data_ptr(), B, A, F,
+                      T, P, R, self._I, int(self._circ), sh)
+            if self._inc:
+                _lib.call("blade_incoherent_detect_ci8", x.data_ptr(), ph.data_ptr(), row, A, F, T, P, R, self._I,
+                          int(self._circ), sh)
+            return result.success
+        pre = _out(self._pre)
         _lib.call("blade_prechannelize_cf16", x.data_ptr(), pre.data_ptr(), A, F, T, P, R, int(self._circ), sh)
         _lib.call("blade_beamform_prepare_detect_tc_cf16", ph.data_ptr(), plan.data_ptr(), pre.data_ptr(),
                   out.data_ptr(), B, A, F * R, T // R, P, self._I, sh)
-        if self._inc:  # beam row B: the incoherent beam through the detector
-            row = out.data_ptr() + B * F * R * (T // (R * self._I)) * 4
+        if self._inc:
             _lib.call("blade_incoherent_detect_cf16", pre.data_ptr(), ph.data_ptr(), row, A, F * R, T // R, P,
                       self._I, sh)
         return result.success
@@ -991,9 +1010,9 @@ class ModeB(Module):
     configures it (mode_b.hh:146-147).  When the chain is Beamformer -> Detector
     alone (rate 1, no circular conversion, no incoherent beam, Stokes-I), it runs
     as one fused launch (tensor cores for CI8 input, FP32 CUDA cores for CF32).
-    CI8 input at rate 2 or 4 with Stokes-I runs the pre-beamformer stages into
-    exact FP16 and the tensor-core chain on the fine channels, plus the detected
-    incoherent beam when enabled (``tensor_cores`` is True).  Elsewhere the
+    CI8 input at rate 2 or 4 with Stokes-I runs on tensor cores with per-fine-channel
+    phasors, plus the detected incoherent beam when enabled (``tensor_cores`` is
+    True).  Elsewhere the
     pre-beamformer stages run as one launch up to rate 4096, and up to 16 beams the
     Beamformer -> Detector pair as another (windows of up to 32 spectra, a power of
     two); what these do not take runs the module kernels in order."""

@@ -310,6 +310,29 @@ BLADE_API int blade_beamform_prepare_detect_tc_cf16(const void* phasors, void* p
                              uint64_t F, uint64_t T, uint64_t P, uint64_t integration,
                              blade_stream_t stream);
 
+/* ---------------------------------------------------------------------------
+ * The same chain from the CI8 block itself, without the fine channels in memory:
+ * split and tensor-core Cast -> Channelizer(rate) -> [Polarizer] -> Beamformer::ATA
+ * -> Detector (Stokes-I) as one call.  in: CI8 [A,F,T,2]; phasors: CF32
+ * [B,A,F*rate,1,2]; plan: scratch of blade_beamform_tc_plan_size(B, A, F*rate, 2)
+ * bytes; out: F32 [B, F*rate, T/(rate*I), 1].  Limits (.._supported() returns 1 when
+ * met): P = 2, A <= 32, rate 4 with B <= 16 or rate 2 with B <= 32, T % 128 == 0,
+ * I a power of two <= 32, rate * I dividing T.  `in` must be ready before the call is
+ * enqueued.
+ * blade_incoherent_detect_ci8: blade_incoherent_detect_cf16 of those fine channels,
+ * out F32 [F*rate, T/(rate*I)]; rate 2 or 4.
+ * ------------------------------------------------------------------------- */
+BLADE_API int blade_modeb_detect_tc_supported(uint64_t B, uint64_t A, uint64_t F, uint64_t T,
+                                    uint64_t P, uint64_t rate, uint64_t integration);
+BLADE_API int blade_modeb_detect_tc(const void* phasors, void* plan, const void* in, void* out,
+                          uint64_t B, uint64_t A, uint64_t F, uint64_t T, uint64_t P,
+                          uint64_t rate, uint64_t integration, int circular,
+                          blade_stream_t stream);
+BLADE_API int blade_incoherent_detect_ci8(const void* in, const void* phasors, void* out,
+                                uint64_t A, uint64_t F, uint64_t T, uint64_t P,
+                                uint64_t rate, uint64_t integration, int circular,
+                                blade_stream_t stream);
+
 /* Incoherent beam of Beamformer::ATA (src/modules/beamformer/beamformer.cu:64-78,
  * square-rooted because the detector follows, mode_b.hh:146-147) through the
  * Stokes-I detector on CF16 [A,F,T,2] voltages: out[f, u] = sum over the window
