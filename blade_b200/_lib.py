@@ -126,6 +126,18 @@ def call(name: str, *args) -> int:
     return st
 
 
+def current_stream():
+    """Handle of the current stream of the current device (None without CUDA).
+
+    Read without building the ``torch.cuda.Stream`` object around it: 0.4 us instead
+    of 4 us, a third of a small module's call."""
+    import torch
+
+    if torch.cuda.is_initialized():
+        return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
+    return torch.cuda.current_stream().cuda_stream if torch.cuda.is_available() else None
+
+
 def u64_array(values):
     arr = (C.c_uint64 * len(values))(*[int(v) for v in values])
     return arr

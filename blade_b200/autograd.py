@@ -44,7 +44,7 @@ def _adjoint(x: torch.Tensor, w: torch.Tensor, path: str = "auto"):
     if path not in _ENTRY:
         raise ValueError(f"path must be one of {sorted(_ENTRY)}")
     _lib.call(_ENTRY[path], x.data_ptr(), w.data_ptr(), grad.data_ptr(), loss.data_ptr(), B, A, F, T, P,
-              torch.cuda.current_stream().cuda_stream)
+              _lib.current_stream())
     return loss[0], grad
 
 
@@ -60,8 +60,9 @@ class StokesLoss(torch.autograd.Function):
     @staticmethod
     def backward(ctx, grad_out):
         (g,) = ctx.saved_tensors
-        # g = dL/d conj(w); torch wants dL/dRe w + i dL/dIm w = 2 g (L is real).
-        return None, (2.0 * grad_out.to(torch.float32)) * g, None
+        # g = dL/d conj(w); torch wants dL/dRe w + i dL/dIm w = 2 g (L is real).  The
+        # scalar takes g's precision in the product.
+        return None, g * (2.0 * grad_out), None
 
 
 def stokes_loss(x: torch.Tensor, w: torch.Tensor, path: str = "auto") -> torch.Tensor:

@@ -31,7 +31,7 @@ _COMPLEX = {"ci8", "cf16", "cf32", "cf64"}
 
 def _stream_handle(stream) -> Optional[int]:
     if stream is None:
-        return torch.cuda.current_stream().cuda_stream if torch.cuda.is_available() else None
+        return _lib.current_stream()
     if isinstance(stream, int):
         return stream
     return stream.cuda_stream
