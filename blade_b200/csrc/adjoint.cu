@@ -402,28 +402,34 @@ __global__ void __launch_bounds__(kB1Threads) adjoint_b1_kernel(const float4* __
 }
 
 // ---- tensor-core path (P = 2, A <= 32, B <= 32, T a multiple of 128) ----------
-// Per CTA one channel f and one chunk of 128-sample tiles, both polarisations; the
-// phases of a tile run in order, separated by barriers:
-//  1. every thread converts its voltages (loaded during the previous tile's
-//     gradient MMAs) into FP16 hi/lo pairs and stores two operand forms:
-//       XF[p][h]  128 rows (sample s) x K = [Re x | Im x] of 32 antennas,
-//       XG[h]     128 rows m = 64 p + 2 a + c (c = 0: Re, 1: Im) x K = 128 samples,
-//     both K-major with the 128-byte swizzle;
+// Per CTA one channel f and one chunk of 128-sample tiles, both polarisations.  Per tile:
+//  1. every thread splits its voltages (loaded during the previous tile) into FP16
+//     hi/lo pairs and stores XF[p][h]: 128 rows (sample s) x K = [Re x | Im x] of 32
+//     antennas, K-major with the 128-byte swizzle;
 //  2. one thread issues the forward y = x w per polarisation against the hi/lo
 //     phasor image of blade_beamform_tc_prepare (its stacked layout: hi and lo
 //     products side by side along N) for x hi and for x lo, FP32 accumulators in
-//     tensor memory;
-//  3. warps 0-3 (lane = sample) read y = hi + lo, add |y|^2 to the loss, split y into
-//     FP16 hi/lo and store YG[h]: 4 NB rows n = 2 NB p + NB c + b x K = 128 samples;
+//     tensor memory, while all store XG[h] from the same registers: 128 rows
+//     m = 64 p + 2 a + c (c = 0: Re, 1: Im) x K = 128 samples;
+//  3. every warp (lane = sample, four warps per polarisation) reads y = hi + lo, adds
+//     |y|^2 to the loss, splits y into FP16 hi/lo and stores YG[h]: 4 NB rows
+//     n = 2 NB p + NB c + b x K = 128 samples;
 //  4. one thread issues G += XG YG^T for the four (x, y) hi/lo combinations: M = 128
 //     rows (both polarisations), N = 4 NB, K = 128, accumulated over the chunk in
-//     tensor memory (the cross-polarisation blocks are computed and never read).
+//     tensor memory (the cross-polarisation blocks are computed and never read), while
+//     the others start the next tile's step 1.
 // At the end lanes 2 a and 2 a + 1 of warp quarter p hold, for every beam, the four
 // real products of (Re x_a, Im x_a) with (Re y_b, Im y_b); one lane shuffle gives
 //   Re G = Re x . Re y + Im x . Im y,   Im G = Re x . Im y - Im x . Re y,
 // and G = sum_t y conj(x) per chunk goes to the partial sums that the two reduction
 // kernels above add in a fixed order.  The phases wait on tcgen05 commits with
 // bounded waits; on expiry the kernel records a status and returns.
+//
+// 28 antennas x 192 channels x 2048 samples, 16 beams: 113 us with the split and the
+// reductions, 224 us when the steps of a tile ran one after the other with XF stores
+// eight to a bank, steps 3 on half of the warps, and one chunk per channel (192 CTAs
+// on 148 SMs); the shorter chunks also halve the gradient's error (7.8e-6 to 4.0e-6:
+// accumulators in tensor memory truncate).
 constexpr int kTcThreads = 256;
 constexpr uint32_t kTcKA = 32;
 constexpr long long kTcBudget = 2000000000ll;
@@ -438,11 +444,13 @@ struct AdjTcArgs {
 
 __device__ unsigned int g_adj_status = 0;
 
+// hi = rn(v), lo = rn(v - hi) of two values as FP16 pairs (v0 in the low half).
 __device__ __forceinline__ uint32_t split_pair(float v0, float v1, uint32_t& lo) {
-    const __half h0 = __float2half_rn(v0), h1 = __float2half_rn(v1);
-    const __half l0 = __float2half_rn(v0 - __half2float(h0)), l1 = __float2half_rn(v1 - __half2float(h1));
-    lo = (uint32_t)__half_as_ushort(l0) | ((uint32_t)__half_as_ushort(l1) << 16);
-    return (uint32_t)__half_as_ushort(h0) | ((uint32_t)__half_as_ushort(h1) << 16);
+    const __half2 h = __floats2half2_rn(v0, v1);
+    const float2 f = __half22float2(h);
+    const __half2 l = __floats2half2_rn(v0 - f.x, v1 - f.y);
+    lo = *reinterpret_cast<const uint32_t*>(&l);
+    return *reinterpret_cast<const uint32_t*>(&h);
 }
 
 // Byte offset of K element k (k even for 4-byte pairs) of `row` in a K-major 128-byte-
@@ -482,13 +490,11 @@ __global__ void __launch_bounds__(kTcThreads, 1) adjoint_tc_kernel(const AdjTcAr
         tmem_alloc(tmem_slot, 512);
         tmem_relinquish();
     }
-    // the channel's phasor image and zero voltage operands (padded antennas stay 0)
+    // the channel's phasor image (every word of the operands is written for each tile)
     {
         const uint4* src = reinterpret_cast<const uint4*>(g.plan + (uint64_t)f * g.img_bytes);
         uint4* dst = reinterpret_cast<uint4*>(img);
         for (uint32_t i = tid; i < g.img_bytes / 16; i += kTcThreads) dst[i] = src[i];
-        uint4* z = reinterpret_cast<uint4*>(xf);
-        for (uint32_t i = tid; i < (4 * 16384 + 2 * 32768) / 16; i += kTcThreads) z[i] = make_uint4(0u, 0u, 0u, 0u);
     }
     fence_proxy_async_smem();
     tc_fence_before();
@@ -499,12 +505,18 @@ __global__ void __launch_bounds__(kTcThreads, 1) adjoint_tc_kernel(const AdjTcAr
     const uint32_t dg = tmem + 256u;           // gradient accumulator, columns 256 .. 256 + 4 NB
     const uint32_t idesc_f = idesc_f16(128, d_cols), idesc_g = idesc_f16(128, 4u * NB);
 
-    // voltages of this thread's tasks: (antenna pair a2, sample pair s2) = (t / 64, t % 64)
+    // This thread's tasks i = 0..3: antennas (a0, a0 + 1) x samples (s0, s0 + 1) of warp block
+    // warp + 8 i (4 antenna octets x 8 groups of 16 samples; lane = 4 antenna pairs x 8
+    // sample pairs).  Stores swap the order of a lane's two samples (XF) or antennas (XG)
+    // in half of the lanes, so that a warp's 32 words always fall in 32 banks.
+    const uint32_t la = lane & 3u, ls = lane >> 2, flip_s = ls >> 2, flip_a = la >> 1;
     float4 xv[4][4];  // [task][(a0, s0), (a0, s0 + 1), (a0 + 1, s0), (a0 + 1, s0 + 1)]
+    auto task_a = [&](int i) { return 8u * ((warp + 8u * i) & 3u) + 2u * la; };
+    auto task_s = [&](int i) { return 16u * ((warp + 8u * i) >> 2) + 2u * ls; };
     auto load = [&](uint32_t tile) {
 #pragma unroll
         for (int i = 0; i < 4; i++) {
-            const uint32_t tk = tid + kTcThreads * i, a0 = 2u * (tk >> 6), s0 = 2u * (tk & 63u);
+            const uint32_t a0 = task_a(i), s0 = task_s(i);
 #pragma unroll
             for (int e = 0; e < 4; e++) {
                 const uint32_t a = a0 + (e >> 1), s = s0 + (e & 1);
@@ -517,59 +529,54 @@ __global__ void __launch_bounds__(kTcThreads, 1) adjoint_tc_kernel(const AdjTcAr
     uint32_t fph = 0, gph = 0;
     bool ok = true;
     if (tile0 < tile1) load(tile0);
-    for (uint32_t tile = tile0; tile < tile1 && ok; tile++) {
-        // the previous tile's gradient MMAs read XF/XG/YG: wait for them
-        if (tile > tile0) {
-            const bool w = mbar_wait(&bars[1], gph, &never, kTcBudget);
-            gph ^= 1;
-            if (!__syncthreads_and(w)) {
-                ok = false;
-                break;
-            }
-            tc_fence_after();
-        }
-        // phase 1: operands
+    for (uint32_t tile = tile0; tile < tile1; tile++) {
+        // the four voltages of each (task, polarisation, component) as FP16 pairs of
+        // samples: [.][0], [1] hi of a0 and a0 + 1, [2], [3] lo
+        uint32_t hv[4][2][2][4];
 #pragma unroll
-        for (int i = 0; i < 4; i++) {
-            const uint32_t tk = tid + kTcThreads * i, a0 = 2u * (tk >> 6), s0 = 2u * (tk & 63u);
-            if (a0 >= kTcKA) continue;
+        for (int i = 0; i < 4; i++)
 #pragma unroll
-            for (int p = 0; p < 2; p++) {
+            for (int p = 0; p < 2; p++)
 #pragma unroll
                 for (int c = 0; c < 2; c++) {
-                    // component (p, c) of the four samples: v[a][s]
-                    float v[2][2];
+                    float v[4];
 #pragma unroll
                     for (int e = 0; e < 4; e++) {
                         const float4 q = xv[i][e];
-                        v[e >> 1][e & 1] = p ? (c ? q.w : q.z) : (c ? q.y : q.x);
+                        v[e] = p ? (c ? q.w : q.z) : (c ? q.y : q.x);
                     }
-                    // XF: row s, K = 32 c + a0 (antennas a0, a0 + 1)
-#pragma unroll
-                    for (int ds = 0; ds < 2; ds++) {
-                        uint32_t lo;
-                        const uint32_t hi = split_pair(v[0][ds], v[1][ds], lo);
-                        const uint32_t off = kmaj_off(s0 + ds, 32u * c + a0, 16384u);
-                        *reinterpret_cast<uint32_t*>(xf + (2 * p + 0) * 16384 + off) = hi;
-                        *reinterpret_cast<uint32_t*>(xf + (2 * p + 1) * 16384 + off) = lo;
-                    }
-                    // XG: row 64 p + 2 a + c, K = s0 (samples s0, s0 + 1)
-#pragma unroll
-                    for (int da = 0; da < 2; da++) {
-                        uint32_t lo;
-                        const uint32_t hi = split_pair(v[da][0], v[da][1], lo);
-                        const uint32_t off = kmaj_off(64u * p + 2u * (a0 + da) + c, s0, 16384u);
-                        *reinterpret_cast<uint32_t*>(xg + off) = hi;
-                        *reinterpret_cast<uint32_t*>(xg + 32768 + off) = lo;
-                    }
+                    hv[i][p][c][0] = split_pair(v[0], v[1], hv[i][p][c][2]);
+                    hv[i][p][c][1] = split_pair(v[2], v[3], hv[i][p][c][3]);
                 }
-            }
+        // XF: row s, K = 32 c + a0 (antennas a0, a0 + 1).  The forward MMAs of the previous
+        // tile have finished; its gradient MMAs, which may still run, read XG and YG.
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const uint32_t a0 = task_a(i), s0 = task_s(i);
+#pragma unroll
+            for (int c = 0; c < 2; c++)
+#pragma unroll
+                for (uint32_t d = 0; d < 2; d++) {
+                    const uint32_t ds = d ^ flip_s, sel = ds ? 0x7632u : 0x5410u;
+                    const uint32_t off = kmaj_off(s0 + ds, 32u * c + a0, 16384u);
+#pragma unroll
+                    for (int p = 0; p < 2; p++)
+#pragma unroll
+                        for (int h = 0; h < 2; h++)
+                            *reinterpret_cast<uint32_t*>(xf + (2 * p + h) * 16384 + off) =
+                                __byte_perm(hv[i][p][c][2 * h], hv[i][p][c][2 * h + 1], sel);
+                }
         }
+        // the next tile's voltages travel through the rest of this one
+        if (tile + 1 < tile1) load(tile + 1);
         fence_proxy_async_smem();
         tc_fence_before();
-        __syncthreads();
+        if (!__syncthreads_and(ok)) {
+            ok = false;
+            break;
+        }
         tc_fence_after();
-        // phase 2: forward, x hi and x lo against the stacked hi/lo image
+        // forward, x hi and x lo against the stacked hi/lo image
         if (tid == 0) {
             const uint64_t wdesc = smem_desc_sw128(smem_u32(img));
             const uint32_t wpol16 = 4u * NB * 8u;  // one polarisation's column block of 4 NB rows
@@ -586,55 +593,67 @@ __global__ void __launch_bounds__(kTcThreads, 1) adjoint_tc_kernel(const AdjTcAr
             }
             mma_commit(&bars[0]);
         }
-        // the next tile's voltages travel while the tensor cores work
-        if (tile + 1 < tile1) load(tile + 1);
-        {
-            const bool w = mbar_wait(&bars[0], fph, &never, kTcBudget);
-            fph ^= 1;
-            if (!__syncthreads_and(w)) {
-                ok = false;
-                break;
-            }
-            tc_fence_after();
+        // XG: row 64 p + 2 a + c, K = s0 (samples s0, s0 + 1), once the previous tile's
+        // gradient MMAs have read it
+        if (tile > tile0) {
+            ok = mbar_wait(&bars[1], gph, &never, kTcBudget) && ok;
+            gph ^= 1;
         }
-        // phase 3: y (lane = sample) -> loss and the YG operand
-        if (warp < 4) {
-            const uint32_t s = 32u * warp + lane;
-            const uint32_t lane_addr = tmem + ((32u * warp) << 16);
-            float lt = 0.f;
-            for (uint32_t p = 0; p < 2; p++) {
-                for (uint32_t b0 = 0; b0 < NB; b0 += 16) {
-                    uint32_t hr[16], hi_[16], lr[16], li[16];
-                    tmem_ld16(lane_addr + p * d_cols + b0, hr);
-                    tmem_ld16(lane_addr + p * d_cols + NB + b0, hi_);
-                    tmem_ld16(lane_addr + p * d_cols + 2 * NB + b0, lr);
-                    tmem_ld16(lane_addr + p * d_cols + 3 * NB + b0, li);
-                    tmem_ld_wait();
 #pragma unroll
-                    for (int e = 0; e < 16; e++) {
-                        const float yr = __uint_as_float(hr[e]) + __uint_as_float(lr[e]);
-                        const float yi = __uint_as_float(hi_[e]) + __uint_as_float(li[e]);
-                        lt = fmaf(yr, yr, fmaf(yi, yi, lt));
-                        const uint32_t b = b0 + e;
+        for (int i = 0; i < 4; i++) {
+            const uint32_t a0 = task_a(i), s0 = task_s(i);
 #pragma unroll
-                        for (int c = 0; c < 2; c++) {
-                            const float v = c ? yi : yr;
-                            const __half h = __float2half_rn(v);
-                            const __half l = __float2half_rn(v - __half2float(h));
-                            const uint32_t off = kmaj_off(2u * NB * p + NB * c + b, s, yblk);
-                            *reinterpret_cast<__half*>(yg + off) = h;
-                            *reinterpret_cast<__half*>(yg + yg_h + off) = l;
-                        }
+            for (int p = 0; p < 2; p++)
+#pragma unroll
+                for (int c = 0; c < 2; c++)
+#pragma unroll
+                    for (uint32_t d = 0; d < 2; d++) {
+                        const uint32_t da = d ^ flip_a;
+                        const uint32_t off = kmaj_off(64u * p + 2u * (a0 + da) + c, s0, 16384u);
+                        *reinterpret_cast<uint32_t*>(xg + off) = da ? hv[i][p][c][1] : hv[i][p][c][0];
+                        *reinterpret_cast<uint32_t*>(xg + 32768 + off) = da ? hv[i][p][c][3] : hv[i][p][c][2];
                     }
+        }
+        ok = mbar_wait(&bars[0], fph, &never, kTcBudget) && ok;
+        fph ^= 1;
+        tc_fence_after();
+        // y of polarisation p (lane = sample) -> loss and the YG operand
+        {
+            const uint32_t q = warp & 3u, p = warp >> 2, s = 32u * q + lane;
+            const uint32_t lane_addr = tmem + ((32u * q) << 16) + p * d_cols;
+            float lt = 0.f;
+            for (uint32_t b0 = 0; b0 < NB; b0 += 16) {
+                uint32_t hr[16], hi_[16], lr[16], li[16];
+                tmem_ld16(lane_addr + b0, hr);
+                tmem_ld16(lane_addr + NB + b0, hi_);
+                tmem_ld16(lane_addr + 2 * NB + b0, lr);
+                tmem_ld16(lane_addr + 3 * NB + b0, li);
+                tmem_ld_wait();
+#pragma unroll
+                for (int e = 0; e < 16; e++) {
+                    const float yr = __uint_as_float(hr[e]) + __uint_as_float(lr[e]);
+                    const float yi = __uint_as_float(hi_[e]) + __uint_as_float(li[e]);
+                    lt = fmaf(yr, yr, fmaf(yi, yi, lt));
+                    uint32_t lo;  // halves (Re, Im)
+                    const uint32_t hi = split_pair(yr, yi, lo);
+                    const uint32_t b = b0 + e;
+                    const uint32_t o_r = kmaj_off(2u * NB * p + b, s, yblk), o_i = kmaj_off(2u * NB * p + NB + b, s, yblk);
+                    *reinterpret_cast<uint16_t*>(yg + o_r) = (uint16_t)hi;
+                    *reinterpret_cast<uint16_t*>(yg + o_i) = (uint16_t)(hi >> 16);
+                    *reinterpret_cast<uint16_t*>(yg + yg_h + o_r) = (uint16_t)lo;
+                    *reinterpret_cast<uint16_t*>(yg + yg_h + o_i) = (uint16_t)(lo >> 16);
                 }
             }
             lsum += (double)lt;
         }
         fence_proxy_async_smem();
         tc_fence_before();
-        __syncthreads();
+        if (!__syncthreads_and(ok)) {
+            ok = false;
+            break;
+        }
         tc_fence_after();
-        // phase 4: G += XG YG^T over the four hi/lo combinations, accumulated over the chunk
+        // G += XG YG^T over the four hi/lo combinations, accumulated over the chunk
         if (tid == 0) {
             for (uint32_t hx = 0; hx < 2; hx++)
                 for (uint32_t hy = 0; hy < 2; hy++) {
@@ -741,6 +760,23 @@ cudaError_t scratch_alloc(void** p, size_t bytes, cudaStream_t s) {
     return cudaMallocFromPoolAsync(p, bytes, pool, s);
 }
 
+// One scratch block per call, handed out in 256-byte aligned pieces in the order of
+// `sizes` (each allocation and each free costs about a microsecond of the call).
+template <int N>
+int scratch_pieces(const char* who, const uint64_t (&sizes)[N], uint8_t* (&pieces)[N], cudaStream_t s) {
+    uint64_t total = 0;
+    for (int i = 0; i < N; i++) total += ceil_div(sizes[i], 256) * 256;
+    void* base = nullptr;
+    const cudaError_t e = scratch_alloc(&base, total, s);
+    if (e != cudaSuccess) return check_cuda(e, who);
+    uint8_t* p = static_cast<uint8_t*>(base);
+    for (int i = 0; i < N; i++) {
+        pieces[i] = p;
+        p += ceil_div(sizes[i], 256) * 256;
+    }
+    return BLADE_SUCCESS;
+}
+
 }  // namespace
 }  // namespace bb
 
@@ -771,21 +807,29 @@ int adjoint_tensor_cores(const void* in, const void* phasors, void* grad, double
     const uint64_t plan_bytes = blade_beamform_tc_plan_size(B, A, F, 2);
     if (plan_bytes != (uint64_t)F * img_bytes) return set_error(BLADE_ASSERTION_ERROR, "%s: image layout", who);
     const uint64_t ntiles = T / 128, Q = B * A;
-    uint64_t nch = (uint64_t)sm_count() / F;  // one CTA per SM (all of tensor memory)
-    if (nch < 1) nch = 1;
-    if (nch > ntiles) nch = ntiles;
-    const uint64_t tpc = (ntiles + nch - 1) / nch;
-    nch = (ntiles + tpc - 1) / tpc;
+    // Chunks per channel: one CTA per SM (all of tensor memory), so the time is the number
+    // of waves of F nch CTAs times a chunk's tiles plus about one and a half tiles of
+    // start-up and final reduction; the fewest chunks among equals.
+    uint64_t nch = 1, tpc = ntiles, best = ~0ull;
+    for (uint64_t n = 1; n <= ntiles && n <= 64; n++) {
+        const uint64_t per = ceil_div(ntiles, n), chunks = ceil_div(ntiles, per);
+        const uint64_t cost = ceil_div(F * chunks, (uint64_t)sm_count()) * (2 * per + 3);
+        if (cost < best) {
+            best = cost;
+            nch = chunks;
+            tpc = per;
+        }
+    }
     const size_t smem = adjoint_tc_smem(NB, img_bytes);
     if (int rc = ensure_smem(reinterpret_cast<const void*>(adjoint_tc_kernel), smem)) return rc;
-    uint8_t* plan = nullptr;
-    float4* gpart = nullptr;
-    double* lpart = nullptr;
-    cudaError_t e = scratch_alloc(reinterpret_cast<void**>(&plan), plan_bytes, s);
-    if (e == cudaSuccess) e = scratch_alloc(reinterpret_cast<void**>(&gpart), F * nch * Q * sizeof(float4), s);
-    if (e == cudaSuccess) e = scratch_alloc(reinterpret_cast<void**>(&lpart), F * nch * sizeof(double), s);
-    int rc = e == cudaSuccess ? BLADE_SUCCESS : check_cuda(e, "blade_beamform_detect_adjoint (scratch)");
-    if (!rc) rc = blade_beamform_tc_prepare(phasors, plan, B, A, F, 2, reinterpret_cast<blade_stream_t>(s));
+    uint8_t* pieces[3];
+    int rc = scratch_pieces("blade_beamform_detect_adjoint (scratch)",
+                            {plan_bytes, F * nch * Q * sizeof(float4), F * nch * sizeof(double)}, pieces, s);
+    if (rc) return rc;
+    uint8_t* plan = pieces[0];
+    float4* gpart = reinterpret_cast<float4*>(pieces[1]);
+    double* lpart = reinterpret_cast<double*>(pieces[2]);
+    rc = blade_beamform_tc_prepare(phasors, plan, B, A, F, 2, reinterpret_cast<blade_stream_t>(s));
     if (!rc) {
         AdjTcArgs g;
         g.x = static_cast<const float4*>(in);
@@ -806,9 +850,7 @@ int adjoint_tensor_cores(const void* in, const void* phasors, void* grad, double
         if (loss) loss_sum_kernel<<<1, 256, 0, s>>>(lpart, (uint32_t)(F * nch), loss);
         rc = check_launch(who);
     }
-    if (plan) cudaFreeAsync(plan, s);
-    if (gpart) cudaFreeAsync(gpart, s);
-    if (lpart) cudaFreeAsync(lpart, s);
+    cudaFreeAsync(plan, s);
     return rc;
 }
 
@@ -859,14 +901,12 @@ extern "C" int blade_beamform_detect_adjoint_f32(const void* in, const void* pha
         // one beam: register-resident kernel, chunks of kB1Samples samples
         const uint64_t nch = (T + kB1Samples - 1) / kB1Samples;
         if (F * nch > 0x7fffffffull) return set_error(BLADE_ERROR, "blade_beamform_detect_adjoint_f32: too many chunks");
-        float4* gpart = nullptr;
-        double* lpart = nullptr;
-        cudaError_t e = scratch_alloc(reinterpret_cast<void**>(&gpart), F * nch * A * sizeof(float4), s);
-        if (e == cudaSuccess) e = scratch_alloc(reinterpret_cast<void**>(&lpart), F * nch * sizeof(double), s);
-        if (e != cudaSuccess) {
-            if (gpart) cudaFreeAsync(gpart, s);
-            return check_cuda(e, "blade_beamform_detect_adjoint (scratch)");
-        }
+        uint8_t* pieces[2];
+        if (int rc = scratch_pieces("blade_beamform_detect_adjoint (scratch)",
+                                    {F * nch * A * sizeof(float4), F * nch * sizeof(double)}, pieces, s))
+            return rc;
+        float4* gpart = reinterpret_cast<float4*>(pieces[0]);
+        double* lpart = reinterpret_cast<double*>(pieces[1]);
         const unsigned grid = (unsigned)(F * nch);
         const float4* x4 = static_cast<const float4*>(in);
         const float2* w2 = static_cast<const float2*>(phasors);
@@ -882,7 +922,6 @@ extern "C" int blade_beamform_detect_adjoint_f32(const void* in, const void* pha
         if (loss) loss_sum_kernel<<<1, 256, 0, s>>>(lpart, (uint32_t)(F * nch), loss);
         const int rc = check_launch("blade_beamform_detect_adjoint");
         cudaFreeAsync(gpart, s);
-        cudaFreeAsync(lpart, s);
         return rc;
     }
     const size_t fast_smem = 16 + (Q + A * (kTA + 1) + B * kTA + kTA) * sizeof(float4) + kTA * sizeof(double);
@@ -899,14 +938,12 @@ extern "C" int blade_beamform_detect_adjoint_f32(const void* in, const void* pha
         if (nch < 1) nch = 1;
         const uint64_t tpc = (ntiles + nch - 1) / nch;
         nch = (ntiles + tpc - 1) / tpc;
-        float4* gpart = nullptr;
-        double* lpart = nullptr;
-        cudaError_t e = scratch_alloc(reinterpret_cast<void**>(&gpart), F * nch * Q * sizeof(float4), s);
-        if (e == cudaSuccess) e = scratch_alloc(reinterpret_cast<void**>(&lpart), F * nch * sizeof(double), s);
-        if (e != cudaSuccess) {
-            if (gpart) cudaFreeAsync(gpart, s);
-            return check_cuda(e, "blade_beamform_detect_adjoint (scratch)");
-        }
+        uint8_t* pieces[2];
+        if (int rc0 = scratch_pieces("blade_beamform_detect_adjoint (scratch)",
+                                    {F * nch * Q * sizeof(float4), F * nch * sizeof(double)}, pieces, s))
+            return rc0;
+        float4* gpart = reinterpret_cast<float4*>(pieces[0]);
+        double* lpart = reinterpret_cast<double*>(pieces[1]);
         const int nacc = Q <= (uint64_t)kTA ? 1 : Q <= 2u * kTA ? 2 : Q <= 4u * kTA ? 4 : 8;
         const void* fn = nacc == 1 ? reinterpret_cast<const void*>(adjoint_chunk_kernel<1>)
                          : nacc == 2 ? reinterpret_cast<const void*>(adjoint_chunk_kernel<2>)
@@ -928,7 +965,6 @@ extern "C" int blade_beamform_detect_adjoint_f32(const void* in, const void* pha
             rc = check_launch("blade_beamform_detect_adjoint");
         }
         cudaFreeAsync(gpart, s);
-        cudaFreeAsync(lpart, s);
         return rc;
     }
     // General path: one CTA per (f, p), loss partials per CTA summed by loss_sum_kernel.
