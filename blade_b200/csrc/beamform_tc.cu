@@ -368,14 +368,14 @@ __device__ __forceinline__ R4Task r2_task(uint32_t wt, uint32_t lane, uint32_t A
 }
 
 template <bool PRE>
-__device__ __forceinline__ void r2_pair_task(const uint8_t* raw, uint32_t rrow, uint8_t* op0, uint8_t* op1,
-                                             const R4Task& t, uint32_t circ) {
+__device__ __forceinline__ void r2_pair_words(const uint2 (&vs)[4], uint8_t* op0, uint8_t* op1, const R4Task& t,
+                                              uint32_t circ) {
     const half2 h2304 = __halves2half2(__ushort_as_half(0x6880), __ushort_as_half(0x6880));  // 2304
     half2 zr[4][2], zi[4][2];  // [antenna][k], halves = (pol 0, pol 1)
 #pragma unroll
     for (uint32_t i = 0; i < 4; i++) {
         if (i < t.nvalid) {
-            const uint2 v = *reinterpret_cast<const uint2*>(raw + t.raw_off + i * rrow);
+            const uint2 v = vs[i];
             const uint32_t w[2] = {v.x ^ 0x80808080u, v.y ^ 0x80808080u};
             half2 re[2], im[2];  // 1152 + x
 #pragma unroll
@@ -408,6 +408,36 @@ __device__ __forceinline__ void r2_pair_task(const uint8_t* raw, uint32_t rrow, 
                 make_uint2(__byte_perm(h2u(zi[0][k]), h2u(zi[1][k]), sel), __byte_perm(h2u(zi[2][k]), h2u(zi[3][k]), sel));
         }
     }
+}
+
+template <bool PRE>
+__device__ __forceinline__ void r2_pair_task(const uint8_t* raw, uint32_t rrow, uint8_t* op0, uint8_t* op1,
+                                             const R4Task& t, uint32_t circ) {
+    uint2 v[4];
+#pragma unroll
+    for (uint32_t i = 0; i < 4; i++)
+        v[i] = i < t.nvalid ? *reinterpret_cast<const uint2*>(raw + t.raw_off + i * rrow) : make_uint2(0u, 0u);
+    r2_pair_words<PRE>(v, op0, op1, t, circ);
+}
+
+// Direct mode at R = 2 (no raw ring, as at R = 1 below): the spectra of a warp-task
+// straight from global memory, one 8-byte load per antenna (16 consecutive spectra of
+// each antenna per warp load, 128 contiguous bytes).
+struct Direct2 {
+    uint32_t t_off, a0;  // first sample of the task's spectrum in the tile, first antenna
+};
+
+__device__ __forceinline__ Direct2 direct2_task(uint32_t wt, uint32_t lane) {
+    const uint32_t s = (wt & 3u) * 16u + (lane & 7u) + ((lane >> 4) << 3);
+    return {2u * s, (2u * (wt >> 2) + ((lane >> 3) & 1u)) * 4u};
+}
+
+__device__ __forceinline__ void direct2_load(const uint32_t* in, uint32_t F, uint32_t T, uint32_t f, uint32_t t0,
+                                             const Direct2& d, uint32_t nvalid, uint2 (&v)[4]) {
+    const uint32_t* row = in + ((uint64_t)d.a0 * F + f) * T + t0 + d.t_off;
+#pragma unroll
+    for (uint32_t i = 0; i < 4; i++)
+        v[i] = i < nvalid ? __ldg(reinterpret_cast<const uint2*>(row + (uint64_t)i * F * T)) : make_uint2(0u, 0u);
 }
 
 // Rate 1 from CF16 voltages (the ModeB path: channelized and polarized on the
@@ -1328,6 +1358,53 @@ __global__ void __launch_bounds__(kThreads, 1) bf_tc_kernel(const TcArgs g, cons
                 }
             }
         }
+        if constexpr (R == 2 && ES == 4 && !PRE) {
+            if (g.direct) {
+                // Pair mode without a raw ring: registers hold the next tile's words, asked for as
+                // soon as this tile's are converted; the tile after that is asked into L2.
+                constexpr uint32_t kMaxTk = kMaxKA / 2 / kConvWarps;
+                const uint32_t ntk = KA / 2 / kConvWarps;
+                const uint32_t* in32 = reinterpret_cast<const uint32_t*>(g.in);
+                R4Task tk[kMaxTk];
+                Direct2 dt[kMaxTk];
+                uint2 v[kMaxTk][4];
+                uint32_t f = (uint32_t)(L0 / tpc), tt = (uint32_t)(L0 % tpc);
+#pragma unroll
+                for (uint32_t i = 0; i < kMaxTk; i++) {
+                    const uint32_t wt = (ct >> 5) + i * kConvWarps;
+                    tk[i] = r2_task(wt, lane, g.A, KA, 0);
+                    dt[i] = direct2_task(wt, lane);
+                    if (i >= ntk) tk[i].nvalid = 0;
+                    if (L0 < L1) direct2_load(in32, g.F, g.T, f, tt * kM, dt[i], tk[i].nvalid, v[i]);
+                }
+                uint32_t as = 0, aph = 0;
+                for (uint64_t L = L0; L < L1; L++) {
+                    if (++tt == tpc) { tt = 0; f++; }
+                    if (!mbar_wait(&a_empty[as + 1], aph ^ 1, abort, kWaitBudget)) { record_abort(abort, 8); break; }
+                    uint8_t* op0 = a_smem + (size_t)as * op_bytes;
+#pragma unroll
+                    for (uint32_t i = 0; i < kMaxTk; i++) {
+                        if (i < ntk) r2_pair_words<false>(v[i], op0, op0 + op_bytes, tk[i], 0);
+                    }
+                    fence_proxy_async_smem();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&a_full[as + 1]);
+                    if (L + 1 < L1) {
+#pragma unroll
+                        for (uint32_t i = 0; i < kMaxTk; i++)
+                            direct2_load(in32, g.F, g.T, f, tt * kM, dt[i], tk[i].nvalid, v[i]);
+                    }
+                    // antenna ct of the tile after next (512 bytes)
+                    if (ct < g.A && L + 2 < L1) {
+                        uint32_t pf = f, pt = tt + 1;
+                        if (pt == tpc) { pt = 0; pf++; }
+                        prefetch_l2_bulk(in32 + ((uint64_t)ct * g.F + pf) * g.T + pt * kM, kM * 4);
+                    }
+                    as += 2;
+                    if (as == AS) { as = 0; aph ^= 1; }
+                }
+            }
+        }
         if (!(R == 4 && split) && !g.direct) {
         // R = 4 pair mode: this warp's warp-tasks (KA / 4 of them over kConvWarps warps),
         // addresses fixed for the kernel
@@ -1659,11 +1736,13 @@ bool tc_shape(uint64_t B, uint64_t A, TcShape& s, uint64_t T = 0, uint32_t es = 
     s.a_stages = as;
     s.r_stages = rs;
     s.smem = fixed + as * op + rs * (size_t)s.raw_bytes;
-    if (T && es == 4 && rate == 1 && as < 4) {
+    if (T && es == 4 && (rate == 1 || rate == 2) && as < 4) {
         // A phasor image this large leaves no room for a raw ring and a build-ahead
-        // operand ring together: at rate 1 the converter threads load the voltages
+        // operand ring together: at rates 1 and 2 the converter threads load the voltages
         // themselves and the shared memory holds operand tile pairs only (two pairs
         // at least, so that the build runs a tile ahead and two issuers alternate).
+        // 42 antennas x 50 channels x 1920 samples, 37 beams, rate 2: 28.0 us with three
+        // operand and two raw stages, 23.9 with direct loads.
         for (uint32_t c : {8u, 4u}) {
             if (fixed + c * op <= limit) {
                 s.direct = 1;
@@ -1701,7 +1780,7 @@ bool tc_apply(TcShape& s, uint64_t A, uint64_t T, uint32_t es, uint64_t rate, co
     s.a_stages = c.a_stages;
     if (c.mode == 1) {
         // direct loads run in pair mode: an even operand ring of at least four stages
-        if (es != 4 || rate != 1 || (c.a_stages & 1u) || c.a_stages < 4u) return false;
+        if (es != 4 || (rate != 1 && rate != 2) || (c.a_stages & 1u) || c.a_stages < 4u) return false;
         s.direct = 1;
         s.raw_tiles = 1;
         s.raw_row = kM * es;
