@@ -7,8 +7,9 @@
 // the 48 KB static limit, and A = B = 64 does not compile) and the block size is
 // capped by the register file at large A.
 //
-// Here up to 16 beams run in the streaming kernel of beamform_stream.cuh.  For more a
-// CTA owns one channel f, a tile of TT = 4 TG consecutive time samples and
+// Here beam voltages come from the streaming kernel of beamform_stream.cuh.  In the
+// tiled kernel below (the fused chain, and antenna counts beyond the other's shared
+// memory) a CTA owns one channel f, a tile of TT = 4 TG consecutive time samples and
 // a tile of BT = 4 (256 / TG) beams.  Thread (tg, bg) accumulates a 4 x 4 register
 // tile: 4 consecutive time samples x 4 beams x P polarisations.  Antennas stream
 // through double-buffered shared memory in chunks of AC = 256 / TG (voltages stored
@@ -339,15 +340,12 @@ int launch_stream_beams(const StreamArgs& g, uint32_t nb, uint32_t ns, cudaStrea
 int beamform_f32_beams(const char* who, const void* in, const float2* ph, void* out, uint64_t B, uint64_t A,
                        uint64_t F, uint64_t T, uint64_t P, const PhLayout& lay, int inc, cudaStream_t s) {
     if (B == 0) return BLADE_SUCCESS;
-    const int tg = pick_tg(B);
-    const uint64_t tiles = ceil_div(T, (uint64_t)tg * 4) * F * ceil_div(B, (uint64_t)(256 / tg) * 4);
-    // Up to 16 beams the voltages are read once or twice and the streaming kernel is
-    // faster at every size measured (1.2x at 16 beams, 1.8x at 8, 2.5x at one); with more
-    // it would read them once per eight beams, which only pays when the tiled kernel
-    // leaves SMs idle (64 beams x 64 antennas x 4 channels x 512 samples: 13.1 against
-    // 17.3 us for one thread per output).
+    // The streaming kernel reads the voltages once per eight beams (from L2 after the first
+    // time) and is faster at every size measured: 2.2 times at 8 beams x 20 antennas, 1.4
+    // at 32 x 28, 1.15 at 64 x 64, 2 and more on small blocks.  The tiled kernel stays for
+    // antenna counts whose weights exceed shared memory.
     uint32_t nb, ns;
-    if ((B <= 16 || tiles < 2ull * sm_count()) && stream_shape(B, A, F, T, P, nb, ns)) {
+    if (stream_shape(B, A, F, T, P, nb, ns)) {
         StreamArgs g{};
         g.in = in;
         g.ph = ph;
@@ -361,6 +359,7 @@ int beamform_f32_beams(const char* who, const void* in, const float2* ph, void* 
         if (int rc = P == 2 ? launch_stream_beams<2>(g, nb, ns, s) : launch_stream_beams<1>(g, nb, ns, s)) return rc;
         return check_launch(who);
     }
+    const int tg = pick_tg(B);
     if (P == 2) dispatch_tg<2, IN_CF32, 0>(tg, in, ph, out, B, A, F, T, 1, s, lay);
     else dispatch_tg<1, IN_CF32, 0>(tg, in, ph, out, B, A, F, T, 1, s, lay);
     if (inc) {
@@ -407,28 +406,26 @@ namespace bb {
 namespace {
 
 // Whether the beams and the incoherent beam run through the detector inside the
-// streaming kernel: windows that a warp closes with lane shuffles, and at most two
-// reads of the voltages (16 beams, 28 antennas x 768 channels x 2048 samples: 467 us
-// against 735 us for the kernels one by one; 8 beams x 20 antennas 1.7 to 2.5 times
-// faster; beyond 16 beams the tiled beamformer reads the voltages less often).
+// streaming kernel: windows that a warp closes with lane shuffles (16 beams, 28
+// antennas x 768 channels x 2048 samples: 396 us against 735 us for the kernels one by
+// one; 8 beams x 20 antennas 2.1 to 5 times faster).
 bool products_shape(uint64_t B, uint64_t A, uint64_t F, uint64_t T, uint64_t P, uint64_t I, uint64_t out_pols,
-                    uint32_t& nb) {
-    uint32_t ns;
-    if (P != 2 || B == 0 || B > 16 || A == 0 || F == 0 || T == 0 || !dims_ok(B, A, F, T)) return false;
+                    uint32_t& nb, uint32_t& ns) {
+    if (P != 2 || B == 0 || A == 0 || F == 0 || T == 0 || !dims_ok(B, A, F, T)) return false;
     if (I == 0 || I > 32 || (I & (I - 1)) != 0 || T % I != 0 || (out_pols != 1 && out_pols != 4)) return false;
-    // one sample per thread: the products' shuffles need the registers of the second
-    return stream_shape(B, A, F, T, P, nb, ns) && stream_smem(nb, 1, A, F, T, P) <= 160 * 1024 &&
-           ceil_div(F * ceil_div(T, 32), kStreamWarps) * ceil_div(B, nb) < (1ull << 31);
+    return stream_shape(B, A, F, T, P, nb, ns);
 }
 
 template <int IN, int OP>
-int launch_products(const StreamArgs& g, uint32_t nb, cudaStream_t s) {
+int launch_products(const StreamArgs& g, uint32_t nb, uint32_t ns, cudaStream_t s) {
+#define BB_PRODUCTS(NBV) (ns == 2 ? launch_stream<2, NBV, 2, IN, OP>(g, s) : launch_stream<2, NBV, 1, IN, OP>(g, s))
     switch (nb) {
-        case 1: return launch_stream<2, 1, 1, IN, OP>(g, s);
-        case 2: return launch_stream<2, 2, 1, IN, OP>(g, s);
-        case 4: return launch_stream<2, 4, 1, IN, OP>(g, s);
-        default: return launch_stream<2, 8, 1, IN, OP>(g, s);
+        case 1: return BB_PRODUCTS(1);
+        case 2: return BB_PRODUCTS(2);
+        case 4: return BB_PRODUCTS(4);
+        default: return BB_PRODUCTS(8);
     }
+#undef BB_PRODUCTS
 }
 
 }  // namespace
@@ -436,8 +433,8 @@ int launch_products(const StreamArgs& g, uint32_t nb, cudaStream_t s) {
 
 extern "C" int blade_beamform_products_supported(uint64_t B, uint64_t A, uint64_t F, uint64_t T, uint64_t P,
                                                  uint64_t integration, uint64_t out_pols) {
-    uint32_t nb;
-    return bb::products_shape(B, A, F, T, P, integration, out_pols, nb) ? 1 : 0;
+    uint32_t nb, ns;
+    return bb::products_shape(B, A, F, T, P, integration, out_pols, nb, ns) ? 1 : 0;
 }
 
 extern "C" int blade_beamform_products_f32(int in_type, const void* in, const void* phasors, void* out, uint64_t B,
@@ -447,11 +444,11 @@ extern "C" int blade_beamform_products_f32(int in_type, const void* in, const vo
     const char* who = "blade_beamform_products_f32";
     if (in_type != BLADE_CF32 && in_type != BLADE_CI8)
         return set_error(BLADE_ERROR, "%s: input type must be CF32 or CI8", who);
-    uint32_t nb;
-    if (!products_shape(B, A, F, T, P, integration, out_pols, nb))
+    uint32_t nb, ns;
+    if (!products_shape(B, A, F, T, P, integration, out_pols, nb, ns))
         return set_error(BLADE_ERROR,
                          "%s: unsupported configuration (B=%llu A=%llu F=%llu T=%llu P=%llu I=%llu out_pols=%llu): "
-                         "needs P = 2, 1 <= B <= 16, I a power of two <= 32 dividing T, 1 or 4 products", who,
+                         "needs P = 2, I a power of two <= 32 dividing T, 1 or 4 products", who,
                          (unsigned long long)B, (unsigned long long)A, (unsigned long long)F, (unsigned long long)T,
                          (unsigned long long)P, (unsigned long long)integration, (unsigned long long)out_pols);
     if (!in || !phasors || !out) return set_error(BLADE_ERROR, "%s: null buffer", who);
@@ -471,9 +468,9 @@ extern "C" int blade_beamform_products_f32(int in_type, const void* in, const vo
     g.lay = ata_layout(A, F, P);
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
     int rc;
-    if (in_type == BLADE_CF32) rc = out_pols == 1 ? launch_products<STREAM_CF32, 1>(g, nb, s)
-                                                  : launch_products<STREAM_CF32, 4>(g, nb, s);
-    else rc = out_pols == 1 ? launch_products<STREAM_CI8, 1>(g, nb, s) : launch_products<STREAM_CI8, 4>(g, nb, s);
+    if (in_type == BLADE_CF32) rc = out_pols == 1 ? launch_products<STREAM_CF32, 1>(g, nb, ns, s)
+                                                  : launch_products<STREAM_CF32, 4>(g, nb, ns, s);
+    else rc = out_pols == 1 ? launch_products<STREAM_CI8, 1>(g, nb, ns, s) : launch_products<STREAM_CI8, 4>(g, nb, ns, s);
     return rc ? rc : check_launch(who);
 }
 

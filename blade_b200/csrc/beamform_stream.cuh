@@ -1,5 +1,5 @@
-// Streaming FP32 beamformer for few beams: voltages go straight from global memory
-// to registers, once per tile of NB beams.
+// Streaming FP32 beamformer: the voltages stream through a private ring in shared
+// memory, once per tile of NB beams.
 //
 //   y[b, f, t, p] = sum_a x[a, f, t, p] w[b, a, f, 0, p]
 // (reference src/modules/beamformer/beamformer.cu:13-79), with the incoherent beam
@@ -9,18 +9,19 @@
 //
 // A warp owns 32 NS consecutive samples of one channel (lane l: samples l + 32 s)
 // and NB beams; a CTA's four warps take consecutive tiles, which may lie in up to
-// four channels when the channels are short.  Each antenna costs NS 16-byte loads
-// per lane (kU antennas in flight ahead of the arithmetic) and NB broadcast reads of
-// its weights from shared memory, which the NS samples share.
+// four channels when the channels are short.  Each lane copies its own samples of the
+// next kDepth - 1 antennas into shared memory (cp.async, read back by the same lane, so
+// no barrier is involved) and reads each antenna's NB weights as broadcasts, which its
+// NS samples share.
 //
-// Bound by the voltage read plus the FP32 pipe (57 % issue, long_scoreboard the
-// top stall): 20 antennas x 192 channels x 8192 samples, 8 beams: 163 us for 705 MB
-// (4.3 TB/s), where staging voltages and weights in shared memory took 288 us
-// behind its barriers (one every two antennas).  Packed FP32x2 arithmetic is no
-// faster (173 us), nor are one sample (165 us) or four beams x four samples (166 us)
-// per thread.  With detection (20 antennas x 6144 channels x 128 samples, 8 beams and
-// the incoherent one, four products): 105 us against 470 us for the tiled kernel,
-// the incoherent kernel and the detector.
+// Bound by the voltage read plus the FP32 pipe: 20 antennas x 192 channels x 8192
+// samples, 8 beams: 128 us for 705 MB (5.5 TB/s).  Staging voltages and weights behind
+// a barrier every two antennas took 288 us, two rounds of register loads 162 (128
+// registers, 15 warps per SM waiting on memory).  Packed FP32x2 arithmetic is no
+// faster, one sample per lane 142, four 135, a ring of four 133, of eight 146.  With
+// detection (20 antennas x 6144 channels x 128 samples, 8 beams and the incoherent one,
+// four products) 93 us against 470 us for the tiled kernel, the incoherent kernel and
+// the detector.
 #pragma once
 
 #include "common.cuh"
@@ -51,30 +52,41 @@ constexpr int kStreamWarps = 4;
 
 enum { STREAM_CF32 = 0, STREAM_CI8 = 1 };
 
+constexpr int kStreamDepth = 6;  // antennas in the ring
+
+// Bytes of one sample (P polarisations) and its values.
 template <int P, int IN>
-__device__ __forceinline__ void stream_load(const void* in, uint64_t i, float2 (&v)[P]) {
-    if constexpr (IN == STREAM_CF32 && P == 2) {
-        const float4 q = ldg_nc_f4(static_cast<const float4*>(in) + i);
-        v[0] = make_float2(q.x, q.y);
-        v[1] = make_float2(q.z, q.w);
-    } else if constexpr (IN == STREAM_CF32) {
-        v[0] = __ldg(static_cast<const float2*>(in) + i);
-    } else {
-        static_assert(P == 2, "CI8 input is dual-polarisation");
-        const float4 q = ci8_f4(__ldg(static_cast<const uint32_t*>(in) + i));
-        v[0] = make_float2(q.x, q.y);
-        v[1] = make_float2(q.z, q.w);
+struct StreamSample {
+    static constexpr int kBytes = IN == STREAM_CI8 ? 4 : 8 * P;
+    static_assert(IN == STREAM_CF32 || P == 2, "CI8 input is dual-polarisation");
+
+    static __device__ __forceinline__ void copy(uint32_t dst, const void* in, uint64_t i) {
+        const char* src = static_cast<const char*>(in) + i * kBytes;
+        if constexpr (kBytes == 16) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+        else asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(dst), "l"(src), "n"(kBytes) : "memory");
     }
-}
+    static __device__ __forceinline__ void read(const unsigned char* p, float2 (&v)[P]) {
+        if constexpr (kBytes == 8) {
+            v[0] = *reinterpret_cast<const float2*>(p);
+        } else {
+            const float4 q = kBytes == 16 ? *reinterpret_cast<const float4*>(p)
+                                          : ci8_f4(*reinterpret_cast<const uint32_t*>(p));
+            v[0] = make_float2(q.x, q.y);
+            v[P - 1] = make_float2(q.z, q.w);
+        }
+    }
+};
 
 // OP = 0: beam voltages CF32 [B (+ 1), F, T, P]; OP = 1 or 4: detected products F32
 // [B (+ 1), F, T / I, OP] (P = 2).
 template <int P, int NB, int NS, int IN, int OP>
-__global__ void __launch_bounds__(kStreamWarps * 32, NB == 8 && NS == 2 ? 4 : 1) bf_stream_kernel(const StreamArgs g) {
-    constexpr int kU = 4 / NS;  // antennas per load round, two rounds in flight
-    extern __shared__ __align__(16) float2 ws[];  // [channel][A padded to kU][NB][P]
+__global__ void __launch_bounds__(kStreamWarps * 32, NB == 8 && NS == 2 ? 5 : 1)
+    bf_stream_kernel(const StreamArgs g) {
+    using Sample = StreamSample<P, IN>;
+    constexpr uint32_t kThreads = kStreamWarps * 32, kSlot = kThreads * Sample::kBytes;
+    extern __shared__ __align__(16) unsigned char stream_smem_raw[];  // ring [kStreamDepth][NS][thread], weights
+    float2* ws = reinterpret_cast<float2*>(stream_smem_raw + kStreamDepth * NS * kSlot);  // [channel][A][NB][P]
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
-    const uint32_t Ap = (g.A + kU - 1) / kU * kU;
     const uint32_t blk = blockIdx.x / g.nbt, b0 = (blockIdx.x - blk * g.nbt) * NB;
     const uint64_t first = (uint64_t)blk * kStreamWarps;
     const uint64_t last = min(first + kStreamWarps, g.tiles) - 1;
@@ -84,36 +96,35 @@ __global__ void __launch_bounds__(kStreamWarps * 32, NB == 8 && NS == 2 ? 4 : 1)
     const uint32_t f = active ? (uint32_t)(tile / g.ntt) : f0;
     const uint32_t t0 = (uint32_t)(tile - (uint64_t)f * g.ntt) * (32 * NS) + lane;
     const uint64_t astride = (uint64_t)g.F * g.T, x0 = (uint64_t)f * g.T + t0;
-    auto load = [&](uint32_t a0, float2 (&x)[kU][NS][P]) {
+    unsigned char* mine = stream_smem_raw + tid * Sample::kBytes;
+    const uint32_t ring = static_cast<uint32_t>(__cvta_generic_to_shared(mine));
+    // antenna a into ring position `at` (an empty group past the last antenna keeps the count)
+    auto fetch = [&](uint32_t a, uint32_t at) {
+        if (active && a < g.A) {
 #pragma unroll
-        for (int u = 0; u < kU; u++)
-#pragma unroll
-            for (int s = 0; s < NS; s++) {
-                if (a0 + u < g.A && t0 + 32 * s < g.T) {
-                    stream_load<P, IN>(g.in, (a0 + u) * astride + x0 + 32 * s, x[u][s]);
-                } else {
-#pragma unroll
-                    for (int p = 0; p < P; p++) x[u][s][p] = make_float2(0.f, 0.f);
-                }
-            }
+            for (int s = 0; s < NS; s++)
+                if (t0 + 32 * s < g.T) Sample::copy(ring + (at * NS + s) * kSlot, g.in, a * astride + x0 + 32 * s);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
     };
-    float2 xa[kU][NS][P], xb[kU][NS][P];
-    // on their way while the weights are gathered (with two samples per thread the
-    // registers held across the gather cost more: 170 against 163 us on the block above)
-    if (NS == 1 && active) load(0, xa);
-    // weights of this CTA's channels, padded beams and antennas zero
-    for (uint32_t r = tid; r < NB * Ap; r += kStreamWarps * 32) {
+#pragma unroll
+    for (uint32_t a = 0; a < kStreamDepth - 1; a++) fetch(a, a);  // on their way while the weights are gathered
+    // weights of this CTA's channels, padded beams zero
+    for (uint32_t r = tid; r < NB * g.A; r += kThreads) {
         const uint32_t a = r / NB, j = r - a * NB;
-        const bool ok = a < g.A && b0 + j < g.B;
+        const bool ok = b0 + j < g.B;
         const float2* src = g.ph + (b0 + j) * g.lay.sb + a * g.lay.sa + (uint64_t)f0 * g.lay.sf;
         for (uint32_t c = 0; c < nch; c++)
 #pragma unroll
             for (int p = 0; p < P; p++)
-                ws[((c * Ap + a) * NB + j) * P + p] = ok ? __ldg(src + c * g.lay.sf + p * g.lay.sp) : make_float2(0.f, 0.f);
+                ws[((c * g.A + a) * NB + j) * P + p] = ok ? __ldg(src + c * g.lay.sf + p * g.lay.sp) : make_float2(0.f, 0.f);
     }
     __syncthreads();
-    if (!active) return;
-    const float2* wc = ws + (size_t)(f - f0) * Ap * NB * P;
+    if (!active) {
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        return;
+    }
+    const float2* wa = ws + (size_t)(f - f0) * g.A * NB * P;
     const bool inc = g.inc != 0 && b0 == 0;
 
     float2 acc[NB][NS][P];
@@ -126,43 +137,40 @@ __global__ void __launch_bounds__(kStreamWarps * 32, NB == 8 && NS == 2 ? 4 : 1)
 #pragma unroll
             for (int j = 0; j < NB; j++) acc[j][s][p] = make_float2(0.f, 0.f);
         }
-    auto mac = [&](uint32_t a0, const float2 (&x)[kU][NS][P]) {
-#pragma unroll
-        for (int u = 0; u < kU; u++) {
-            const float2* wa = wc + (size_t)(a0 + u) * NB * P;
-#pragma unroll
-            for (int j = 0; j < NB; j++) {
-                float2 w[P];
-                if constexpr (P == 2) {
-                    const float4 q = *reinterpret_cast<const float4*>(wa + j * P);
-                    w[0] = make_float2(q.x, q.y);
-                    w[1] = make_float2(q.z, q.w);
-                } else {
-                    w[0] = wa[j];
-                }
-#pragma unroll
-                for (int s = 0; s < NS; s++)
-#pragma unroll
-                    for (int p = 0; p < P; p++) {
-                        const float2 xv = x[u][s][p];
-                        acc[j][s][p].x = fmaf(xv.x, w[p].x, fmaf(-xv.y, w[p].y, acc[j][s][p].x));
-                        acc[j][s][p].y = fmaf(xv.x, w[p].y, fmaf(xv.y, w[p].x, acc[j][s][p].y));
-                        if (j == 0 && inc) {
-                            const float re = xv.x * w[p].x - xv.y * w[p].y, im = xv.x * w[p].y + xv.y * w[p].x;
-                            pw[s][p] += re * re + im * im;
-                        }
-                    }
-            }
-        }
-    };
-    if (NS != 1) load(0, xa);
+    uint32_t at = 0, to = kStreamDepth - 1;
 #pragma unroll 1
-    for (uint32_t a0 = 0; a0 < g.A; a0 += 2 * kU) {
-        if (a0 + kU < g.A) load(a0 + kU, xb);
-        mac(a0, xa);
-        if (a0 + kU >= g.A) break;
-        if (a0 + 2 * kU < g.A) load(a0 + 2 * kU, xa);
-        mac(a0 + kU, xb);
+    for (uint32_t a = 0; a < g.A; a++) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(kStreamDepth - 2) : "memory");
+        float2 x[NS][P];
+#pragma unroll
+        for (int s = 0; s < NS; s++) Sample::read(mine + (at * NS + s) * kSlot, x[s]);
+        fetch(a + kStreamDepth - 1, to);
+        to = at;
+        if (++at == kStreamDepth) at = 0;
+#pragma unroll
+        for (int j = 0; j < NB; j++) {
+            float2 w[P];
+            if constexpr (P == 2) {
+                const float4 q = *reinterpret_cast<const float4*>(wa + j * P);
+                w[0] = make_float2(q.x, q.y);
+                w[1] = make_float2(q.z, q.w);
+            } else {
+                w[0] = wa[j];
+            }
+#pragma unroll
+            for (int s = 0; s < NS; s++)
+#pragma unroll
+                for (int p = 0; p < P; p++) {
+                    const float2 xv = x[s][p];
+                    acc[j][s][p].x = fmaf(xv.x, w[p].x, fmaf(-xv.y, w[p].y, acc[j][s][p].x));
+                    acc[j][s][p].y = fmaf(xv.x, w[p].y, fmaf(xv.y, w[p].x, acc[j][s][p].y));
+                    if (j == 0 && inc) {
+                        const float re = xv.x * w[p].x - xv.y * w[p].y, im = xv.x * w[p].y + xv.y * w[p].x;
+                        pw[s][p] += re * re + im * im;
+                    }
+                }
+        }
+        wa += NB * P;
     }
 
     if constexpr (OP == 0) {
@@ -196,11 +204,26 @@ __global__ void __launch_bounds__(kStreamWarps * 32, NB == 8 && NS == 2 ? 4 : 1)
                 v[2] = x.x * y.x + x.y * y.y;  // Re x conj(y)
                 v[3] = x.y * y.x - x.x * y.y;  // Im x conj(y)
             }
+            const bool stored = t0 + 32 * s < g.T;
+            float* d = out + (((uint64_t)row * g.F + f) * U + ((t0 + 32 * s) >> g.log_integ)) * OP;
+            if constexpr (OP == 4) {
+                // windows of four and more: two halving exchanges leave one product per lane
+                if (I >= 4) {
+                    const bool hi = lane & 1u, up = lane & 2u;
+                    const float s0 = hi ? v[0] : v[2], s1 = hi ? v[1] : v[3];
+                    float k0 = hi ? v[2] : v[0], k1 = hi ? v[3] : v[1];
+                    k0 += __shfl_xor_sync(0xffffffffu, s0, 1);
+                    k1 += __shfl_xor_sync(0xffffffffu, s1, 1);
+                    float k = (up ? k1 : k0) + __shfl_xor_sync(0xffffffffu, up ? k0 : k1, 2);
+                    for (uint32_t o = 4; o < I; o <<= 1) k += __shfl_xor_sync(0xffffffffu, k, o);
+                    if (stored && (lane & (I - 1u)) < 4) d[2 * (lane & 1u) + ((lane >> 1) & 1u)] = k;
+                    return;
+                }
+            }
             for (uint32_t o = 1; o < I; o <<= 1)
 #pragma unroll
                 for (int q = 0; q < OP; q++) v[q] += __shfl_xor_sync(0xffffffffu, v[q], o);
-            if ((lane & (I - 1u)) == 0 && t0 + 32 * s < g.T) {
-                float* d = out + (((uint64_t)row * g.F + f) * U + ((t0 + 32 * s) >> g.log_integ)) * OP;
+            if ((lane & (I - 1u)) == 0 && stored) {
                 if constexpr (OP == 4) stg_f4(d, make_float4(v[0], v[1], v[2], v[3]));
                 else d[0] = v[0];
             }
@@ -216,18 +239,19 @@ __global__ void __launch_bounds__(kStreamWarps * 32, NB == 8 && NS == 2 ? 4 : 1)
     }
 }
 
-inline size_t stream_smem(uint64_t nb, uint64_t ns, uint64_t A, uint64_t F, uint64_t T, uint64_t P) {
-    const uint64_t kU = 4 / ns, Ap = (A + kU - 1) / kU * kU, ntt = ceil_div(T, 32 * ns);
+inline size_t stream_smem(uint64_t nb, uint64_t ns, uint64_t A, uint64_t F, uint64_t T, uint64_t P,
+                          uint64_t sample_bytes) {
+    const uint64_t ntt = ceil_div(T, 32 * ns);
     // channels that a CTA's consecutive tiles can touch
     uint64_t nch = ntt % kStreamWarps == 0 ? 1 : 1 + ceil_div(kStreamWarps - 1, ntt);
     if (nch > F) nch = F;
-    return nch * Ap * nb * P * sizeof(float2);
+    return kStreamDepth * ns * kStreamWarps * 32 * sample_bytes + nch * A * nb * P * sizeof(float2);
 }
 
 // Beams and samples per thread.  Eight beams share each voltage load and two samples
 // each weight read as long as every SM still gets eight warps; below that, fewer, so
 // that a small block spreads over the SMs (20 antennas x 96 channels x 256 samples,
-// 8 beams with the incoherent beam: 8.8 us against 17.3 us for one thread per
+// 8 beams with the incoherent beam: 8.5 us against 17.3 us for one thread per
 // output).  False: the weights do not fit in shared memory.
 inline bool stream_shape(uint64_t B, uint64_t A, uint64_t F, uint64_t T, uint64_t P, uint32_t& nb, uint32_t& ns) {
     nb = B > 4 ? 8 : B > 2 ? 4 : (uint32_t)B;
@@ -235,8 +259,8 @@ inline bool stream_shape(uint64_t B, uint64_t A, uint64_t F, uint64_t T, uint64_
     const uint64_t want = 8ull * sm_count();
     if (F * ceil_div(T, 64) * ceil_div(B, nb) < want) ns = 1;
     while (nb > 2 && F * ceil_div(T, 32 * ns) * ceil_div(B, nb) < want) nb /= 2;
-    while (nb > 1 && stream_smem(nb, ns, A, F, T, P) > 160 * 1024) nb /= 2;
-    return stream_smem(nb, ns, A, F, T, P) <= 160 * 1024 &&
+    while (nb > 1 && stream_smem(nb, ns, A, F, T, P, 16) > 160 * 1024) nb /= 2;
+    return stream_smem(nb, ns, A, F, T, P, 16) <= 160 * 1024 &&
            ceil_div(F * ceil_div(T, 32 * ns), kStreamWarps) * ceil_div(B, nb) < (1ull << 31);
 }
 
@@ -245,7 +269,7 @@ int launch_stream(StreamArgs g, cudaStream_t s) {
     g.ntt = (uint32_t)ceil_div(g.T, 32 * NS);
     g.tiles = (uint64_t)g.F * g.ntt;
     g.nbt = (uint32_t)ceil_div(g.B, NB);
-    const size_t smem = stream_smem(NB, NS, g.A, g.F, g.T, P);
+    const size_t smem = stream_smem(NB, NS, g.A, g.F, g.T, P, StreamSample<P, IN>::kBytes);
     const auto fn = bf_stream_kernel<P, NB, NS, IN, OP>;
     if (int rc = ensure_smem(reinterpret_cast<const void*>(fn), smem)) return rc;
     fn<<<(unsigned)(ceil_div(g.tiles, kStreamWarps) * g.nbt), kStreamWarps * 32, smem, s>>>(g);

@@ -1013,9 +1013,9 @@ class ModeB(Module):
     CI8 input at rate 2 or 4 with Stokes-I runs on tensor cores with per-fine-channel
     phasors, plus the detected incoherent beam when enabled (``tensor_cores`` is
     True).  Elsewhere the
-    pre-beamformer stages run as one launch up to rate 4096, and up to 16 beams the
-    Beamformer -> Detector pair as another (windows of up to 32 spectra, a power of
-    two); what these do not take runs the module kernels in order."""
+    pre-beamformer stages run as one launch up to rate 4096 and the Beamformer ->
+    Detector pair as another (windows of up to 32 spectra, a power of two); what
+    these do not take runs the module kernels in order."""
 
     taint = Taint.CONSUMER | Taint.PRODUCER
 

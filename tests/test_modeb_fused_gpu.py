@@ -47,7 +47,7 @@ def type_of(it):
 
 @pytest.mark.parametrize("it,A,F,T,B,I,OP,inc", [
     ("cf32", 1, 1, 1, 1, 1, 1, 1), ("cf32", 5, 3, 96, 2, 32, 4, 1), ("ci8", 20, 7, 130, 8, 2, 4, 0),
-    ("cf32", 28, 500, 64, 16, 4, 4, 1), ("ci8", 9, 2, 1000, 9, 8, 1, 1), ("cf32", 42, 6, 4096, 4, 16, 4, 0)])
+    ("cf32", 28, 500, 64, 16, 4, 4, 1), ("ci8", 9, 2, 1000, 9, 8, 1, 1), ("cf32", 42, 6, 4096, 4, 16, 4, 0), ("cf32", 7, 40, 1024, 35, 8, 4, 1)])
 def test_products_match_the_oracle(cuda, it, A, F, T, B, I, OP, inc):
     xh, w = voltages(it, (A, F, T, 2), A + T), crand(np.random.default_rng(B), (B, A, F, 1, 2))
     n = (B + inc) * F * (T // I) * OP
@@ -66,7 +66,8 @@ def test_products_match_the_oracle(cuda, it, A, F, T, B, I, OP, inc):
 def test_products_refuse_what_the_detector_pair_must_run(cuda):
     ok = _lib.load().blade_beamform_products_supported
     assert ok(16, 28, 64, 1024, 2, 32, 4) == 1
-    for B, T, P, I, OP in [(17, 1024, 2, 4, 4), (8, 1024, 1, 4, 4), (8, 1024, 2, 64, 4), (8, 1024, 2, 3, 1),
+    assert ok(100, 28, 64, 1024, 2, 1, 1) == 1
+    for B, T, P, I, OP in [(0, 1024, 2, 4, 4), (8, 1024, 1, 4, 4), (8, 1024, 2, 64, 4), (8, 1024, 2, 3, 1),
                            (8, 1022, 2, 4, 1), (8, 1024, 2, 4, 2), (8, 1024, 2, 0, 1)]:
         assert ok(B, 28, 64, T, P, I, OP) == 0
 

@@ -1,6 +1,6 @@
 """GPU: the FP32 beamformer's streaming kernel at the edges of its tiles (32 samples
-per warp and slot, four warps per CTA over up to four channels, 1 to 8 beams and 2 or
-4 antennas per round) against the FP64 oracle.
+per warp and slot, four warps per CTA over up to four channels, 1 to 8 beams,
+6 antennas in flight) against the FP64 oracle.
 
 Tolerance: each output sums 2 A products of two FP32 roundings each, so its error
 is below (2 A + 2) 2^-24 of the sum of magnitudes, under 1e-5 for A <= 42 by a wide
@@ -26,6 +26,8 @@ TOL = 1e-5
     (7, 40, 2049, 2, 9, True, True),    # nine beams: a second beam tile with one beam
     (42, 16, 8192, 2, 16, False, False),
     (28, 3, 256, 2, 40, True, False),   # many beams of a small block
+    (6, 150, 700, 2, 66, True, True),   # many beam tiles, the last with two beams
+    (13, 300, 130, 1, 17, False, False),
     (200, 2, 64, 2, 5, False, False),   # weights beyond the default shared memory
 ])
 def test_streaming_beamformer(cuda, A, F, T, P, B, inc, sq):
