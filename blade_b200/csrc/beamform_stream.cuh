@@ -15,12 +15,14 @@
 // NS samples share.
 //
 // Bound by the voltage read plus the FP32 pipe: 20 antennas x 192 channels x 8192
-// samples, 8 beams: 128 us for 705 MB (5.5 TB/s).  Staging voltages and weights behind
+// samples, 8 beams: 122 us for 705 MB (5.8 TB/s); 130 when each copy computed its
+// address from the antenna and tested its sample again.  Staging voltages and weights behind
 // a barrier every two antennas took 288 us, two rounds of register loads 162 (128
 // registers, 15 warps per SM waiting on memory).  Packed FP32x2 arithmetic is no
-// faster, one sample per lane 142, four 135, a ring of four 133, of eight 146.  With
+// faster; one sample per lane, four, a ring of four or of eight are 2 to 12 % slower, and
+// so are several tiles per warp (spills) and a loop unrolled to the ring (128).  With
 // detection (20 antennas x 6144 channels x 128 samples, 8 beams and the incoherent one,
-// four products) 93 us against 470 us for the tiled kernel, the incoherent kernel and
+// four products) 88 us against 470 us for the tiled kernel, the incoherent kernel and
 // the detector.
 #pragma once
 
@@ -98,26 +100,31 @@ __global__ void __launch_bounds__(kStreamWarps * 32, NB == 8 && NS == 2 ? 5 : 1)
     const uint64_t astride = (uint64_t)g.F * g.T, x0 = (uint64_t)f * g.T + t0;
     unsigned char* mine = stream_smem_raw + tid * Sample::kBytes;
     const uint32_t ring = static_cast<uint32_t>(__cvta_generic_to_shared(mine));
-    // antenna a into ring position `at` (an empty group past the last antenna keeps the count)
-    auto fetch = [&](uint32_t a, uint32_t at) {
-        if (active && a < g.A) {
+    // antenna a, at src, into the ring position at `dst` (an empty group past the last
+    // antenna keeps the count)
+    bool in_row[NS];
 #pragma unroll
-            for (int s = 0; s < NS; s++)
-                if (t0 + 32 * s < g.T) Sample::copy(ring + (at * NS + s) * kSlot, g.in, a * astride + x0 + 32 * s);
-        }
+    for (int s = 0; s < NS; s++) in_row[s] = active && t0 + 32 * s < g.T;
+    const char* src = static_cast<const char*>(g.in) + x0 * Sample::kBytes;
+    auto fetch = [&](uint32_t a, uint32_t dst) {
+#pragma unroll
+        for (int s = 0; s < NS; s++)
+            if (in_row[s] && a < g.A) Sample::copy(dst + s * kSlot, src, 32 * s);
+        src += astride * Sample::kBytes;
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
 #pragma unroll
-    for (uint32_t a = 0; a < kStreamDepth - 1; a++) fetch(a, a);  // on their way while the weights are gathered
+    for (uint32_t a = 0; a < kStreamDepth - 1; a++)  // on their way while the weights are gathered
+        fetch(a, ring + a * NS * kSlot);
     // weights of this CTA's channels, padded beams zero
     for (uint32_t r = tid; r < NB * g.A; r += kThreads) {
         const uint32_t a = r / NB, j = r - a * NB;
         const bool ok = b0 + j < g.B;
-        const float2* src = g.ph + (b0 + j) * g.lay.sb + a * g.lay.sa + (uint64_t)f0 * g.lay.sf;
+        const float2* wsrc = g.ph + (b0 + j) * g.lay.sb + a * g.lay.sa + (uint64_t)f0 * g.lay.sf;
         for (uint32_t c = 0; c < nch; c++)
 #pragma unroll
             for (int p = 0; p < P; p++)
-                ws[((c * g.A + a) * NB + j) * P + p] = ok ? __ldg(src + c * g.lay.sf + p * g.lay.sp) : make_float2(0.f, 0.f);
+                ws[((c * g.A + a) * NB + j) * P + p] = ok ? __ldg(wsrc + c * g.lay.sf + p * g.lay.sp) : make_float2(0.f, 0.f);
     }
     __syncthreads();
     if (!active) {
@@ -137,16 +144,17 @@ __global__ void __launch_bounds__(kStreamWarps * 32, NB == 8 && NS == 2 ? 5 : 1)
 #pragma unroll
             for (int j = 0; j < NB; j++) acc[j][s][p] = make_float2(0.f, 0.f);
         }
-    uint32_t at = 0, to = kStreamDepth - 1;
+    uint32_t at = 0, to = (kStreamDepth - 1) * NS * kSlot;
 #pragma unroll 1
     for (uint32_t a = 0; a < g.A; a++) {
         asm volatile("cp.async.wait_group %0;" ::"n"(kStreamDepth - 2) : "memory");
         float2 x[NS][P];
 #pragma unroll
-        for (int s = 0; s < NS; s++) Sample::read(mine + (at * NS + s) * kSlot, x[s]);
-        fetch(a + kStreamDepth - 1, to);
+        for (int s = 0; s < NS; s++) Sample::read(mine + at + s * kSlot, x[s]);
+        fetch(a + kStreamDepth - 1, ring + to);
         to = at;
-        if (++at == kStreamDepth) at = 0;
+        at += NS * kSlot;
+        if (at == kStreamDepth * NS * kSlot) at = 0;
 #pragma unroll
         for (int j = 0; j < NB; j++) {
             float2 w[P];
