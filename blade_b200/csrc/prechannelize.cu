@@ -202,9 +202,11 @@ extern "C" int blade_incoherent_detect_cf16(const void* in, const void* phasors,
 // reads 32 x 4 R consecutive bytes of an antenna, four antennas in flight), the
 // rate-R fftshifted transform and the circular basis in registers (exact integers),
 // |x|^2 |w[0]|^2 summed over antennas and polarisations, windows closed with lane
-// shuffles.  A 28-antenna block of 176 MB at R = 4: 50 us (FP32 pipe 58 % busy, 93
-// instructions per antenna and spectrum), where the kernel above reads 352 MB of fine
-// channels in 57; transforming in FP32 instead of FP16 pairs took 52.
+// shuffles.  A 28-antenna block of 176 MB at R = 4: 45 us (bound by the FP32
+// pipe: transforms, conversions and squares), where the kernel above reads 352 MB of fine
+// channels in 57; 48 with CTAs of 256 threads, which close their last wave later, and 51
+// when each load also computed its address from the antenna; transforming in FP32
+// instead of FP16 pairs was 4 % slower.
 namespace bb {
 namespace {
 
@@ -242,8 +244,10 @@ __device__ __forceinline__ void fine_channels(const uint32_t (&w)[R], H2 (&z)[R]
     }
 }
 
+constexpr uint32_t kIncThreads = 128;
+
 template <int R, bool CIRC>
-__global__ void __launch_bounds__(256) incoherent_detect_ci8_kernel(const uint32_t* __restrict__ x,
+__global__ void __launch_bounds__(kIncThreads) incoherent_detect_ci8_kernel(const uint32_t* __restrict__ x,
                                                                     const float2* __restrict__ w0,
                                                                     float* __restrict__ out, uint32_t A, uint32_t F,
                                                                     uint32_t S, uint32_t I) {
@@ -258,7 +262,8 @@ __global__ void __launch_bounds__(256) incoherent_detect_ci8_kernel(const uint32
     auto load = [&](uint32_t a0, uint32_t (&w)[kAhead][R]) {
 #pragma unroll
         for (uint32_t u = 0; u < kAhead; u++)
-            if (a0 + u < A) load_spectrum<R>(src + (a0 + u) * astride, w[u]);
+            if (a0 + u < A) load_spectrum<R>(src + u * astride, w[u]);
+        src += kAhead * astride;
     };
     load(0, wa);
     for (uint32_t i = threadIdx.x; i < A * R; i += blockDim.x) {
@@ -271,6 +276,7 @@ __global__ void __launch_bounds__(256) incoherent_detect_ci8_kernel(const uint32
     float2 acc[R];
 #pragma unroll
     for (int k = 0; k < R; k++) acc[k] = make_float2(0.f, 0.f);
+    const float2* g = gw;
     auto sum = [&](uint32_t a0, const uint32_t (&w)[kAhead][R]) {
 #pragma unroll
         for (uint32_t u = 0; u < kAhead; u++) {
@@ -285,9 +291,10 @@ __global__ void __launch_bounds__(256) incoherent_detect_ci8_kernel(const uint32
                     re = make_float2(r.x - i.y, r.x + i.y);
                     im = make_float2(i.x + r.y, i.x - r.y);
                 }
-                acc[k] = __ffma2_rn(__ffma2_rn(re, re, __fmul2_rn(im, im)), gw[(a0 + u) * R + k], acc[k]);
+                acc[k] = __ffma2_rn(__ffma2_rn(re, re, __fmul2_rn(im, im)), g[u * R + k], acc[k]);
             }
         }
+        g += kAhead * R;
     };
     for (uint32_t a0 = 0; a0 < A; a0 += 2 * kAhead) {
         load(a0 + kAhead, wb);
@@ -323,12 +330,12 @@ extern "C" int blade_incoherent_detect_ci8(const void* in, const void* phasors, 
         return set_error(BLADE_ERROR, "%s: misaligned buffer", who);
     const size_t smem = A * rate * sizeof(float2);
     const uint32_t S = (uint32_t)(T / rate);
-    const dim3 grid((unsigned)ceil_div(S, 256), (unsigned)F);
+    const dim3 grid((unsigned)ceil_div(S, kIncThreads), (unsigned)F);
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
     const auto fn = rate == 4 ? (circular ? incoherent_detect_ci8_kernel<4, true> : incoherent_detect_ci8_kernel<4, false>)
                               : (circular ? incoherent_detect_ci8_kernel<2, true> : incoherent_detect_ci8_kernel<2, false>);
     if (int rc = ensure_smem(reinterpret_cast<const void*>(fn), smem)) return rc;
-    fn<<<grid, 256, smem, st>>>(static_cast<const uint32_t*>(in), static_cast<const float2*>(phasors),
+    fn<<<grid, kIncThreads, smem, st>>>(static_cast<const uint32_t*>(in), static_cast<const float2*>(phasors),
                                 static_cast<float*>(out), (uint32_t)A, (uint32_t)F, S, (uint32_t)integration);
     return check_launch(who);
 }
