@@ -651,7 +651,8 @@ __global__ void __launch_bounds__(kPairThreads8, 1) fft8192_pair_kernel(const fl
 // The inter-step twiddles sit in the row step, whose CTA needs 256 of them per k1 for
 // all its units: each is one sincospif, rounded once.
 //
-// Bound by HBM behind the workspace round trip: the spectrometer's 64 channels x 16
+// Bound by instruction issue and the shared-memory exchanges (blocks whose workspace
+// stays in L2 take as long per channel): the spectrometer's 64 channels x 16
 // spectra (CI8 in, windows of 8) 531 us for 2.45 GB (4.6 TB/s), 796 us for one
 // transform per thread group with three shared-memory passes per step and twiddle
 // recurrences.  The next group's input is asked for while a group is transformed (551 us
