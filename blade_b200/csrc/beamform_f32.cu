@@ -7,9 +7,9 @@
 // the 48 KB static limit, and A = B = 64 does not compile) and the block size is
 // capped by the register file at large A.
 //
-// Here beam voltages come from the streaming kernel of beamform_stream.cuh.  In the
-// tiled kernel below (the fused chain, and antenna counts beyond the other's shared
-// memory) a CTA owns one channel f, a tile of TT = 4 TG consecutive time samples and
+// Here beam voltages come from the streaming kernel of beamform_stream.cuh, those of the
+// smallest blocks from a kernel of one thread per output.  In the tiled kernel of the
+// fused chain a CTA owns one channel f, a tile of TT = 4 TG consecutive time samples and
 // a tile of BT = 4 (256 / TG) beams.  Thread (tg, bg) accumulates a 4 x 4 register
 // tile: 4 consecutive time samples x 4 beams x P polarisations.  Antennas stream
 // through double-buffered shared memory in chunks of AC = 256 / TG (voltages stored
@@ -290,6 +290,34 @@ __global__ void __launch_bounds__(256) incoherent_kernel(const float2* __restric
     }
 }
 
+// Blocks of a few microseconds: one thread per (beam, channel, sample) and all
+// polarisations, antennas in order, nothing staged.  Bound by latency: the loads of a few
+// antennas are in flight at a time and every beam re-reads the voltages from L2.  Same
+// arithmetic per output as the streaming kernel.
+template <int P>
+__global__ void __launch_bounds__(256) bf32_small_kernel(const float2* __restrict__ in,
+                                                         const float2* __restrict__ phasors, float2* __restrict__ out,
+                                                         uint32_t A, uint32_t F, uint32_t T, const PhLayout ph) {
+    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x, f = blockIdx.y, b = blockIdx.z;
+    if (t >= T) return;
+    float2 acc[P];
+#pragma unroll
+    for (int p = 0; p < P; p++) acc[p] = make_float2(0.f, 0.f);
+    const float2* x = in + ((uint64_t)f * T + t) * P;
+    const float2* w = phasors + b * ph.sb + (uint64_t)f * ph.sf;
+    for (uint32_t a = 0; a < A; a++) {
+#pragma unroll
+        for (int p = 0; p < P; p++) {
+            const float2 xv = __ldg(x + (uint64_t)a * F * T * P + p), wv = __ldg(w + a * ph.sa + p * ph.sp);
+            acc[p].x = fmaf(xv.x, wv.x, fmaf(-xv.y, wv.y, acc[p].x));
+            acc[p].y = fmaf(xv.x, wv.y, fmaf(xv.y, wv.x, acc[p].y));
+        }
+    }
+    float2* o = out + (((uint64_t)b * F + f) * T + t) * P;
+#pragma unroll
+    for (int p = 0; p < P; p++) o[p] = acc[p];
+}
+
 template <int P, int TG, int IN, int R>
 void launch_bf(const void* in, const float2* ph, void* out, uint64_t B, uint64_t A, uint64_t F, uint64_t T,
                uint64_t integ, cudaStream_t s, const PhLayout& lay) {
@@ -335,43 +363,49 @@ int launch_stream_beams(const StreamArgs& g, uint32_t nb, uint32_t ns, cudaStrea
 #undef BB_STREAM
 }
 
+// Whether bf32_small_kernel takes a block: its launch has no ring to fill and no weights to
+// gather, which is worth 0.2 to 0.7 us while its CTAs are resident at once.
+//   Two polarisations: up to 4 antennas (192 samples, 8 beams: 1.8 us against 2.2 streamed),
+//   up to 8 at half of the warps an SM holds (2.0 against 2.5; one beam 4.9 against 5.4 at all
+//   of them); with 16 the antennas' serial loads already cost more (0.73 to 0.99 of its time
+//   streamed).
+//   One polarisation: half of the warps and 48 MB of voltages, which stay in L2 for the beams
+//   that re-read them (1.0 to 1.3 times the speed at 96 to 256 antennas; at 60 MB and more
+//   the ring is up to 1.6 times ahead), and one beam, which re-reads none, at more warps than
+//   that (64 antennas x 192 x 1024: 14.0 us against 17.4; 1024 antennas: 243 against 286).
+bool small_shape(uint64_t B, uint64_t A, uint64_t F, uint64_t T, uint64_t P) {
+    const uint64_t sms = (uint64_t)sm_count(), warps = B * F * ceil_div(T, 32);
+    if (B * F * ceil_div(T, 256) > 8 * sms) return false;
+    const bool half = warps <= 32 * sms;
+    if (P == 2) return A <= (B == 1 ? 8 : 4) || (A <= 8 && half);
+    return A <= 4 || (half ? A * F * T * sizeof(float2) <= 48u << 20 : B == 1);
+}
+
 // Beams 0..B-1 of the plain FP32 beamformer for a phasor layout, and with inc the
 // incoherent beam of beam 0's weights (1 sum of powers, 2 its root).
 int beamform_f32_beams(const char* who, const void* in, const float2* ph, void* out, uint64_t B, uint64_t A,
                        uint64_t F, uint64_t T, uint64_t P, const PhLayout& lay, int inc, cudaStream_t s) {
     if (B == 0) return BLADE_SUCCESS;
-    // The streaming kernel reads the voltages once per eight beams (from L2 after the first
-    // time) and is faster at every size measured: 2.2 times at 8 beams x 20 antennas, 1.4
-    // at 32 x 28, 1.15 at 64 x 64, 2 and more on small blocks.  The tiled kernel stays for
-    // antenna counts whose weights exceed shared memory.
-    uint32_t nb, ns;
-    if (stream_shape(B, A, F, T, P, nb, ns)) {
-        StreamArgs g{};
-        g.in = in;
-        g.ph = ph;
-        g.out = out;
-        g.B = (uint32_t)B;
-        g.A = (uint32_t)A;
-        g.F = (uint32_t)F;
-        g.T = (uint32_t)T;
-        g.inc = (uint32_t)inc;
-        g.lay = lay;
-        if (int rc = P == 2 ? launch_stream_beams<2>(g, nb, ns, s) : launch_stream_beams<1>(g, nb, ns, s)) return rc;
+    if (!inc && small_shape(B, A, F, T, P)) {
+        const dim3 grid((unsigned)ceil_div(T, 256), (unsigned)F, (unsigned)B);
+        const auto fn = P == 2 ? bf32_small_kernel<2> : bf32_small_kernel<1>;
+        fn<<<grid, 256, 0, s>>>(static_cast<const float2*>(in), ph, static_cast<float2*>(out), (uint32_t)A,
+                                (uint32_t)F, (uint32_t)T, lay);
         return check_launch(who);
     }
-    const int tg = pick_tg(B);
-    if (P == 2) dispatch_tg<2, IN_CF32, 0>(tg, in, ph, out, B, A, F, T, 1, s, lay);
-    else dispatch_tg<1, IN_CF32, 0>(tg, in, ph, out, B, A, F, T, 1, s, lay);
-    if (inc) {
-        const float2* x = static_cast<const float2*>(in);
-        float2* y = static_cast<float2*>(out);
-        if (P == 2)
-            incoherent_kernel<2><<<grid_for(F * T, 256), 256, 0, s>>>(x, ph, y, (uint32_t)B, (uint32_t)A, (uint32_t)F,
-                                                                     (uint32_t)T, inc == 2);
-        else
-            incoherent_kernel<1><<<grid_for(F * T, 256), 256, 0, s>>>(x, ph, y, (uint32_t)B, (uint32_t)A, (uint32_t)F,
-                                                                     (uint32_t)T, inc == 2);
-    }
+    uint32_t nb, ns;
+    if (!stream_shape(B, F, T, nb, ns)) return set_error(BLADE_ERROR, "%s: dimensions out of range", who);
+    StreamArgs g{};
+    g.in = in;
+    g.ph = ph;
+    g.out = out;
+    g.B = (uint32_t)B;
+    g.A = (uint32_t)A;
+    g.F = (uint32_t)F;
+    g.T = (uint32_t)T;
+    g.inc = (uint32_t)inc;
+    g.lay = lay;
+    if (int rc = P == 2 ? launch_stream_beams<2>(g, nb, ns, s) : launch_stream_beams<1>(g, nb, ns, s)) return rc;
     return check_launch(who);
 }
 
@@ -413,7 +447,7 @@ bool products_shape(uint64_t B, uint64_t A, uint64_t F, uint64_t T, uint64_t P, 
                     uint32_t& nb, uint32_t& ns) {
     if (P != 2 || B == 0 || A == 0 || F == 0 || T == 0 || !dims_ok(B, A, F, T)) return false;
     if (I == 0 || I > 32 || (I & (I - 1)) != 0 || T % I != 0 || (out_pols != 1 && out_pols != 4)) return false;
-    return stream_shape(B, A, F, T, P, nb, ns);
+    return stream_shape(B, F, T, nb, ns);
 }
 
 template <int IN, int OP>

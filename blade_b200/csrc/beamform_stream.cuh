@@ -46,6 +46,7 @@ struct StreamArgs {
     uint32_t inc;        // 0 none, 1 sum of powers, 2 its square root
     uint32_t nbt;        // beam tiles, innermost in the grid (they read the same voltages)
     uint32_t ntt;        // time tiles per channel
+    uint32_t chunk;      // antennas whose weights are in shared memory at a time
     uint64_t tiles;      // F * ntt
     PhLayout lay;
 };
@@ -81,13 +82,17 @@ struct StreamSample {
 
 // OP = 0: beam voltages CF32 [B (+ 1), F, T, P]; OP = 1 or 4: detected products F32
 // [B (+ 1), F, T / I, OP] (P = 2).
-template <int P, int NB, int NS, int IN, int OP>
-__global__ void __launch_bounds__(kStreamWarps * 32, NB == 8 && NS == 2 ? 5 : 1)
+// CHUNKED: the antennas' weights do not fit beside enough CTAs per SM and pass through
+// shared memory g.chunk antennas at a time (a barrier on either side of each gather); the
+// plain kernel holds them all, and the loop over chunks would cost it registers (36 bytes
+// of spills at eight beams and two samples).
+template <int P, int NB, int NS, int IN, int OP, bool CHUNKED>
+__global__ void __launch_bounds__(kStreamWarps * 32, NB == 8 && NS == 2 ? (CHUNKED ? 4 : 5) : 1)
     bf_stream_kernel(const StreamArgs g) {
     using Sample = StreamSample<P, IN>;
     constexpr uint32_t kThreads = kStreamWarps * 32, kSlot = kThreads * Sample::kBytes;
     extern __shared__ __align__(16) unsigned char stream_smem_raw[];  // ring [kStreamDepth][NS][thread], weights
-    float2* ws = reinterpret_cast<float2*>(stream_smem_raw + kStreamDepth * NS * kSlot);  // [channel][A][NB][P]
+    float2* ws = reinterpret_cast<float2*>(stream_smem_raw + kStreamDepth * NS * kSlot);  // [channel][chunk][NB][P]
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
     const uint32_t blk = blockIdx.x / g.nbt, b0 = (blockIdx.x - blk * g.nbt) * NB;
     const uint64_t first = (uint64_t)blk * kStreamWarps;
@@ -116,22 +121,29 @@ __global__ void __launch_bounds__(kStreamWarps * 32, NB == 8 && NS == 2 ? 5 : 1)
 #pragma unroll
     for (uint32_t a = 0; a < kStreamDepth - 1; a++)  // on their way while the weights are gathered
         fetch(a, ring + a * NS * kSlot);
-    // weights of this CTA's channels, padded beams zero
-    for (uint32_t r = tid; r < NB * g.A; r += kThreads) {
-        const uint32_t a = r / NB, j = r - a * NB;
-        const bool ok = b0 + j < g.B;
-        const float2* wsrc = g.ph + (b0 + j) * g.lay.sb + a * g.lay.sa + (uint64_t)f0 * g.lay.sf;
-        for (uint32_t c = 0; c < nch; c++)
+    // weights of this CTA's channels and of antennas a0 to a1, padded beams zero
+    const uint32_t held = CHUNKED ? g.chunk : g.A;
+    auto gather = [&](uint32_t a0, uint32_t a1) {
+#pragma unroll 4
+        for (uint32_t r = tid; r < NB * (a1 - a0); r += kThreads) {
+            const uint32_t a = r / NB, j = r - a * NB;
+            const bool ok = b0 + j < g.B;
+            const float2* wsrc = g.ph + (b0 + j) * g.lay.sb + (a0 + a) * g.lay.sa + (uint64_t)f0 * g.lay.sf;
+            for (uint32_t c = 0; c < nch; c++)
 #pragma unroll
-            for (int p = 0; p < P; p++)
-                ws[((c * g.A + a) * NB + j) * P + p] = ok ? __ldg(wsrc + c * g.lay.sf + p * g.lay.sp) : make_float2(0.f, 0.f);
+                for (int p = 0; p < P; p++)
+                    ws[((c * held + a) * NB + j) * P + p] = ok ? __ldg(wsrc + c * g.lay.sf + p * g.lay.sp) : make_float2(0.f, 0.f);
+        }
+        __syncthreads();
+    };
+    if constexpr (!CHUNKED) {
+        gather(0, g.A);
+        if (!active) {
+            asm volatile("cp.async.wait_all;" ::: "memory");
+            return;
+        }
     }
-    __syncthreads();
-    if (!active) {
-        asm volatile("cp.async.wait_all;" ::: "memory");
-        return;
-    }
-    const float2* wa = ws + (size_t)(f - f0) * g.A * NB * P;
+    const float2* wa = ws + (size_t)(f - f0) * held * NB * P;
     const bool inc = g.inc != 0 && b0 == 0;
 
     float2 acc[NB][NS][P];
@@ -145,8 +157,7 @@ __global__ void __launch_bounds__(kStreamWarps * 32, NB == 8 && NS == 2 ? 5 : 1)
             for (int j = 0; j < NB; j++) acc[j][s][p] = make_float2(0.f, 0.f);
         }
     uint32_t at = 0, to = (kStreamDepth - 1) * NS * kSlot;
-#pragma unroll 1
-    for (uint32_t a = 0; a < g.A; a++) {
+    auto antenna = [&](uint32_t a) {
         asm volatile("cp.async.wait_group %0;" ::"n"(kStreamDepth - 2) : "memory");
         float2 x[NS][P];
 #pragma unroll
@@ -179,6 +190,25 @@ __global__ void __launch_bounds__(kStreamWarps * 32, NB == 8 && NS == 2 ? 5 : 1)
                 }
         }
         wa += NB * P;
+    };
+    if constexpr (!CHUNKED) {
+#pragma unroll 1
+        for (uint32_t a = 0; a < g.A; a++) antenna(a);
+    } else {
+#pragma unroll 1
+        for (uint32_t a0 = 0; a0 < g.A; a0 += g.chunk) {
+            const uint32_t a1 = min(a0 + g.chunk, g.A);
+            if (a0) __syncthreads();  // every warp has read the chunk before
+            gather(a0, a1);
+            if (!active) continue;
+            wa = ws + (size_t)(f - f0) * held * NB * P;
+#pragma unroll 1
+            for (uint32_t a = a0; a < a1; a++) antenna(a);
+        }
+        if (!active) {
+            asm volatile("cp.async.wait_all;" ::: "memory");
+            return;
+        }
     }
 
     if constexpr (OP == 0) {
@@ -247,29 +277,24 @@ __global__ void __launch_bounds__(kStreamWarps * 32, NB == 8 && NS == 2 ? 5 : 1)
     }
 }
 
-inline size_t stream_smem(uint64_t nb, uint64_t ns, uint64_t A, uint64_t F, uint64_t T, uint64_t P,
-                          uint64_t sample_bytes) {
-    const uint64_t ntt = ceil_div(T, 32 * ns);
-    // channels that a CTA's consecutive tiles can touch
-    uint64_t nch = ntt % kStreamWarps == 0 ? 1 : 1 + ceil_div(kStreamWarps - 1, ntt);
-    if (nch > F) nch = F;
-    return kStreamDepth * ns * kStreamWarps * 32 * sample_bytes + nch * A * nb * P * sizeof(float2);
+// Channels that a CTA's consecutive tiles (from a multiple of kStreamWarps on) can touch.
+inline uint64_t stream_channels(uint64_t ntt, uint64_t F) {
+    const uint64_t nch = ntt == 1 ? kStreamWarps : ntt % kStreamWarps == 0 ? 1 : 2;
+    return nch < F ? nch : F;
 }
 
 // Beams and samples per thread.  Eight beams share each voltage load and two samples
 // each weight read as long as every SM still gets eight warps; below that, fewer, so
 // that a small block spreads over the SMs (20 antennas x 96 channels x 256 samples,
 // 8 beams with the incoherent beam: 8.5 us against 17.3 us for one thread per
-// output).  False: the weights do not fit in shared memory.
-inline bool stream_shape(uint64_t B, uint64_t A, uint64_t F, uint64_t T, uint64_t P, uint32_t& nb, uint32_t& ns) {
+// output).  False: more CTAs than a grid holds.
+inline bool stream_shape(uint64_t B, uint64_t F, uint64_t T, uint32_t& nb, uint32_t& ns) {
     nb = B > 4 ? 8 : B > 2 ? 4 : (uint32_t)B;
     ns = 2;
     const uint64_t want = 8ull * sm_count();
     if (F * ceil_div(T, 64) * ceil_div(B, nb) < want) ns = 1;
     while (nb > 2 && F * ceil_div(T, 32 * ns) * ceil_div(B, nb) < want) nb /= 2;
-    while (nb > 1 && stream_smem(nb, ns, A, F, T, P, 16) > 160 * 1024) nb /= 2;
-    return stream_smem(nb, ns, A, F, T, P, 16) <= 160 * 1024 &&
-           ceil_div(F * ceil_div(T, 32 * ns), kStreamWarps) * ceil_div(B, nb) < (1ull << 31);
+    return ceil_div(F * ceil_div(T, 32 * ns), kStreamWarps) * ceil_div(B, nb) < (1ull << 31);
 }
 
 template <int P, int NB, int NS, int IN, int OP>
@@ -277,10 +302,21 @@ int launch_stream(StreamArgs g, cudaStream_t s) {
     g.ntt = (uint32_t)ceil_div(g.T, 32 * NS);
     g.tiles = (uint64_t)g.F * g.ntt;
     g.nbt = (uint32_t)ceil_div(g.B, NB);
-    const size_t smem = stream_smem(NB, NS, g.A, g.F, g.T, P, StreamSample<P, IN>::kBytes);
-    const auto fn = bf_stream_kernel<P, NB, NS, IN, OP>;
+    const uint64_t ctas = ceil_div(g.tiles, kStreamWarps) * g.nbt, per_sm = ceil_div(ctas, (uint64_t)sm_count());
+    const size_t ring = kStreamDepth * NS * kStreamWarps * 32 * StreamSample<P, IN>::kBytes;
+    const size_t antenna = stream_channels(g.ntt, g.F) * NB * P * sizeof(float2);
+    // Weights beside the ring so that the CTAs an SM gets, four at most, are resident at once:
+    // held in whole they left two CTAs at 512 antennas and one from 768 on (eight beams, two
+    // polarisations).  768 antennas x 170 channels x 1024 samples, 16 beams: 2010 us held in
+    // whole, 957 in chunks (1357 for 4 x 4 register tiles staged behind a barrier); 2048 antennas,
+    // 64 channels, 64 beams: 7920, 3430 (and 4057).
+    const size_t room = 224 * 1024 / (per_sm < 4 ? per_sm : 4) - ring;
+    const bool chunked = g.A * antenna > room;
+    g.chunk = chunked ? (uint32_t)(room / antenna) : g.A;
+    const size_t smem = ring + g.chunk * antenna;
+    const auto fn = chunked ? bf_stream_kernel<P, NB, NS, IN, OP, true> : bf_stream_kernel<P, NB, NS, IN, OP, false>;
     if (int rc = ensure_smem(reinterpret_cast<const void*>(fn), smem)) return rc;
-    fn<<<(unsigned)(ceil_div(g.tiles, kStreamWarps) * g.nbt), kStreamWarps * 32, smem, s>>>(g);
+    fn<<<(unsigned)ctas, kStreamWarps * 32, smem, s>>>(g);
     return BLADE_SUCCESS;
 }
 

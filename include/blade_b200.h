@@ -117,8 +117,7 @@ BLADE_API int blade_beamform_meerkat_f32(const void* in, const void* phasors, vo
  *   out F32 [B+inc, F, T/I, out_pols] = blade_detect(blade_beamform_f32(in, ..., sqrt))
  * in: CF32 or CI8 (cast exactly) [A,F,T,2]; phasors: CF32 [B,A,F,1,2]; out_pols 1 or 4.
  * Limits (blade_beamform_products_supported() returns 1 when met): P = 2, B >= 1,
- * I a power of two <= 32 dividing T, and a few channels' weights of one beam in
- * shared memory (A up to two thousand).
+ * I a power of two <= 32 dividing T.
  * Composes src/modules/beamformer/beamformer.cu:13-79 and src/modules/detector/
  * detector.cu:7-51 as Bundles::ATA::ModeB chains them (mode_b.hh:146-199).
  * ------------------------------------------------------------------------- */
