@@ -183,110 +183,63 @@ __global__ void __launch_bounds__(256, 2) bf32_kernel(const void* __restrict__ v
     }
 
     const uint32_t tb = t0 + tg * 4;  // first of this thread's 4 samples
-    if constexpr (R == 0) {
-        // Beam voltages, CF32 [B, F, T, P].
-        float2* out = static_cast<float2*>(vout);
+    // Stokes-I of the rate-R channelized beams, integrated over `integ` spectra.
+    constexpr int NS = 4 / R;  // spectra held by this thread
+    float* out = static_cast<float*>(vout);
+    const uint32_t U = T / (R * integ);
+    const uint32_t s0 = tb / R;  // first spectrum index of this thread
 #pragma unroll
-        for (int j = 0; j < 4; j++) {
-            const uint32_t b = b0 + bg * 4 + j;
-            if (b >= B) continue;
+    for (int j = 0; j < 4; j++) {
+        const uint32_t b = b0 + bg * 4 + j;
+        float S[NS][R];
 #pragma unroll
-            for (int i = 0; i < 4; i++) {
-                const uint32_t t = tb + i;
-                if (t >= T) continue;
-                float2* o = out + ((uint64_t)(b * (uint64_t)F + f) * T + t) * P;
-                if (P == 2) stg_f4(o, make_float4(acc[i][j][0].x, acc[i][j][0].y, acc[i][j][P - 1].x,
-                                                  acc[i][j][P - 1].y));
-                else o[0] = acc[i][j][0];
+        for (int q = 0; q < NS; q++) {
+#pragma unroll
+            for (int k = 0; k < R; k++) S[q][k] = 0.f;
+#pragma unroll
+            for (int p = 0; p < P; p++) {
+                if (R == 1) {
+                    S[q][0] += pw(acc[q][j][p]);
+                } else if (R == 2) {
+                    const float2 y0 = acc[2 * q][j][p], y1 = acc[2 * q + 1][j][p];
+                    S[q][0] += pw(csub(y0, y1));
+                    S[q][R - 1] += pw(cadd(y0, y1));
+                } else {
+                    const float2 y0 = acc[0][j][p], y1 = acc[1][j][p], y2 = acc[2][j][p], y3 = acc[3][j][p];
+                    const float2 e02 = cadd(y0, y2), d02 = csub(y0, y2);
+                    const float2 e13 = cadd(y1, y3), d13 = csub(y1, y3);
+                    S[q][0] += pw(csub(e02, e13));                 // y0 - y1 + y2 - y3
+                    S[q][R > 1 ? 1 : 0] += pw(cadd(d02, cmuli(d13)));  // y0 + i y1 - y2 - i y3
+                    S[q][R > 2 ? 2 : 0] += pw(cadd(e02, e13));     // y0 + y1 + y2 + y3
+                    S[q][R > 3 ? 3 : 0] += pw(csub(d02, cmuli(d13)));  // y0 - i y1 - y2 + i y3
+                }
             }
         }
-    } else {
-        // Stokes-I of the rate-R channelized beams, integrated over `integ` spectra.
-        constexpr int NS = 4 / R;  // spectra held by this thread
-        float* out = static_cast<float*>(vout);
-        const uint32_t U = T / (R * integ);
-        const uint32_t s0 = tb / R;  // first spectrum index of this thread
-#pragma unroll
-        for (int j = 0; j < 4; j++) {
-            const uint32_t b = b0 + bg * 4 + j;
-            float S[NS][R];
-#pragma unroll
-            for (int q = 0; q < NS; q++) {
-#pragma unroll
-                for (int k = 0; k < R; k++) S[q][k] = 0.f;
-#pragma unroll
-                for (int p = 0; p < P; p++) {
-                    if (R == 1) {
-                        S[q][0] += pw(acc[q][j][p]);
-                    } else if (R == 2) {
-                        const float2 y0 = acc[2 * q][j][p], y1 = acc[2 * q + 1][j][p];
-                        S[q][0] += pw(csub(y0, y1));
-                        S[q][R - 1] += pw(cadd(y0, y1));
-                    } else {
-                        const float2 y0 = acc[0][j][p], y1 = acc[1][j][p], y2 = acc[2][j][p], y3 = acc[3][j][p];
-                        const float2 e02 = cadd(y0, y2), d02 = csub(y0, y2);
-                        const float2 e13 = cadd(y1, y3), d13 = csub(y1, y3);
-                        S[q][0] += pw(csub(e02, e13));                 // y0 - y1 + y2 - y3
-                        S[q][R > 1 ? 1 : 0] += pw(cadd(d02, cmuli(d13)));  // y0 + i y1 - y2 - i y3
-                        S[q][R > 2 ? 2 : 0] += pw(cadd(e02, e13));     // y0 + y1 + y2 + y3
-                        S[q][R > 3 ? 3 : 0] += pw(csub(d02, cmuli(d13)));  // y0 - i y1 - y2 + i y3
-                    }
-                }
-            }
-            if ((uint32_t)NS >= integ) {
-                // Whole windows inside the thread.
-                const uint32_t nw = NS / integ;
-                for (uint32_t v = 0; v < nw; v++) {
-#pragma unroll
-                    for (int k = 0; k < R; k++) {
-                        float sum = 0.f;
-                        for (uint32_t q = v * integ; q < (v + 1) * integ; q++) sum += S[q][k];
-                        const uint32_t u = s0 / integ + v;
-                        if (b < B && u < U) out[((uint64_t)(b * (uint64_t)F + f) * R + k) * U + u] = sum;
-                    }
-                }
-            } else {
-                // Window spans g = integ / NS adjacent lanes (power of two <= 32).
-                const uint32_t g = integ / NS;
+        if ((uint32_t)NS >= integ) {
+            // Whole windows inside the thread.
+            const uint32_t nw = NS / integ;
+            for (uint32_t v = 0; v < nw; v++) {
 #pragma unroll
                 for (int k = 0; k < R; k++) {
                     float sum = 0.f;
-#pragma unroll
-                    for (int q = 0; q < NS; q++) sum += S[q][k];
-                    for (uint32_t o = 1; o < g; o <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-                    const uint32_t u = s0 / integ;
-                    if ((tg % g) == 0 && b < B && u < U) out[((uint64_t)(b * (uint64_t)F + f) * R + k) * U + u] = sum;
+                    for (uint32_t q = v * integ; q < (v + 1) * integ; q++) sum += S[q][k];
+                    const uint32_t u = s0 / integ + v;
+                    if (b < B && u < U) out[((uint64_t)(b * (uint64_t)F + f) * R + k) * U + u] = sum;
                 }
             }
-        }
-    }
-}
-
-// Incoherent beam: out[B, f, t, p] = ([sqrt] sum_a |x[a,f,t,p] w[0,a,f,0,p]|^2, 0)
-// (reference src/modules/beamformer/beamformer.cu:64-78).
-template <int P>
-__global__ void __launch_bounds__(256) incoherent_kernel(const float2* __restrict__ in,
-                                                         const float2* __restrict__ phasors, float2* __restrict__ out,
-                                                         uint32_t B, uint32_t A, uint32_t F, uint32_t T, int do_sqrt) {
-    const uint64_t n = (uint64_t)F * T;
-    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
-        const uint64_t f = i / T;
-        float acc[P];
+        } else {
+            // Window spans g = integ / NS adjacent lanes (power of two <= 32).
+            const uint32_t g = integ / NS;
 #pragma unroll
-        for (int p = 0; p < P; p++) acc[p] = 0.f;
-        for (uint32_t a = 0; a < A; a++) {
+            for (int k = 0; k < R; k++) {
+                float sum = 0.f;
 #pragma unroll
-            for (int p = 0; p < P; p++) {
-                const float2 x = in[((uint64_t)a * F * T + i) * P + p];
-                const float2 w = phasors[((uint64_t)a * F + f) * P + p];
-                const float re = x.x * w.x - x.y * w.y, im = x.x * w.y + x.y * w.x;
-                acc[p] += re * re + im * im;
+                for (int q = 0; q < NS; q++) sum += S[q][k];
+                for (uint32_t o = 1; o < g; o <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+                const uint32_t u = s0 / integ;
+                if ((tg % g) == 0 && b < B && u < U) out[((uint64_t)(b * (uint64_t)F + f) * R + k) * U + u] = sum;
             }
         }
-#pragma unroll
-        for (int p = 0; p < P; p++)
-            out[((uint64_t)B * F * T + i) * P + p] = make_float2(do_sqrt ? sqrtf(acc[p]) : acc[p], 0.f);
     }
 }
 
