@@ -875,10 +875,13 @@ __global__ void __launch_bounds__(k65Threads, 2) fft256_rows_kernel(const float4
 constexpr size_t k65ColsSmem = 4096 * sizeof(float4) + 240 * sizeof(float2);
 
 // Consecutive k1 per CTA of the row step: the largest power of two with at most 16
-// units, so that short blocks still store whole sectors.
-inline uint32_t rows_kk(uint32_t Su) {
+// units, so that short blocks still store whole sectors, that leaves at least `ctas` CTAs:
+// one per SM with the detector, whose window sums take longest (one channel and spectrum,
+// Stokes-I: 8.9 us, 13.0 with 16 units whatever the grid), half of that for spectra (one row
+// and spectrum of two polarisations: 7.5 us, 9.9 with 16 units, 8.3 at one CTA per SM).
+inline uint32_t rows_kk(uint32_t Su, uint64_t rows, uint64_t ctas) {
     uint32_t kk = 1;
-    while (2 * kk * Su <= 16) kk *= 2;
+    while (2 * kk * Su <= 16 && rows * (128 / kk) >= ctas) kk *= 2;
     return kk;
 }
 
@@ -1025,7 +1028,7 @@ extern "C" int blade_channelize(const void* in, void* out, void* workspace, uint
         return set_error(BLADE_ERROR, "blade_channelize: rate %llu has a prime factor above 61", (unsigned long long)rate);
     float2* ws = static_cast<float2*>(workspace);
     if (N1 == 256 && N2 == 256 && S * P <= 32 && aligned16(workspace)) {
-        const uint32_t S32 = (uint32_t)S, Su = P == 2 ? S32 : (S32 + 1) / 2, kk = rows_kk(Su);
+        const uint32_t S32 = (uint32_t)S, Su = P == 2 ? S32 : (S32 + 1) / 2, kk = rows_kk(Su, A * F, sm_count() / 2);
         const uint64_t rows = A * F, cap = (uint64_t)sm_count() * 2, g1 = rows * Su * 16, g2 = rows * (256 / kk);
         const unsigned n1 = (unsigned)(g1 < cap ? g1 : cap), n2 = (unsigned)(g2 < cap ? g2 : cap);
         const size_t sm2 = rows_smem(kk);
@@ -1180,7 +1183,7 @@ int spectrometer_launch(int in_type, const void* in, int out_type, void* out, vo
                         const uint32_t (&per_sm)[2], cudaStream_t s) {
     const uint64_t S = T / 65536;
     float4* ws = static_cast<float4*>(workspace);
-    const uint32_t S32 = (uint32_t)S, I32 = (uint32_t)integration, kk = rows_kk(S32);
+    const uint32_t S32 = (uint32_t)S, I32 = (uint32_t)integration, kk = rows_kk(S32, A * F, sm_count());
     const uint64_t rows = A * F, g1 = rows * S * 16, g2 = rows * (256 / kk);
     const uint64_t cap1 = (uint64_t)sm_count() * per_sm[0], cap2 = (uint64_t)sm_count() * per_sm[1];
     const unsigned grid1 = (unsigned)(g1 < cap1 ? g1 : cap1), grid2 = (unsigned)(g2 < cap2 ? g2 : cap2);
