@@ -19,6 +19,7 @@
 // kernel.
 #include <mutex>
 
+#include "adjoint_chunks.cuh"
 #include "common.cuh"
 #include "tc_ptx.cuh"
 
@@ -807,19 +808,8 @@ int adjoint_tensor_cores(const void* in, const void* phasors, void* grad, double
     const uint64_t plan_bytes = blade_beamform_tc_plan_size(B, A, F, 2);
     if (plan_bytes != (uint64_t)F * img_bytes) return set_error(BLADE_ASSERTION_ERROR, "%s: image layout", who);
     const uint64_t ntiles = T / 128, Q = B * A;
-    // Chunks per channel: one CTA per SM (all of tensor memory), so the time is the number
-    // of waves of F nch CTAs times a chunk's tiles plus about one and a half tiles of
-    // start-up and final reduction; the fewest chunks among equals.
-    uint64_t nch = 1, tpc = ntiles, best = ~0ull;
-    for (uint64_t n = 1; n <= ntiles && n <= 64; n++) {
-        const uint64_t per = ceil_div(ntiles, n), chunks = ceil_div(ntiles, per);
-        const uint64_t cost = ceil_div(F * chunks, (uint64_t)sm_count()) * (2 * per + 3);
-        if (cost < best) {
-            best = cost;
-            nch = chunks;
-            tpc = per;
-        }
-    }
+    uint64_t nch, tpc;
+    adjoint_chunks(F, ntiles, (uint64_t)sm_count(), nch, tpc);
     const size_t smem = adjoint_tc_smem(NB, img_bytes);
     if (int rc = ensure_smem(reinterpret_cast<const void*>(adjoint_tc_kernel), smem)) return rc;
     uint8_t* pieces[3];
