@@ -33,7 +33,8 @@ def _stream(stream):
 
 
 def tensor_core(B, A, F, T, rate=1, integration=1, P=2, stream=None) -> dict:
-    """Tunes the tensor-core chain (blade_beamform_detect_tc family) for one shape."""
+    """Tunes the tensor-core chain (blade_beamform_detect_tc family) for one shape, and for
+    a small block the launch that splits its phasors itself (last key word 5)."""
     _lib.call("blade_beamform_detect_tc_autotune", B, A, F, T, P, rate, integration, _stream(stream))
     return query(TC, (B, A, F, T, P, rate, integration, 4))
 

@@ -202,7 +202,7 @@ bool tc_shape(uint64_t B, uint64_t A, TcShape& s, uint64_t T = 0, uint32_t es = 
 }
 
 // A launch choice of the chain: mode 0 = raw ring of TMA tiles, 1 = converter
-// threads load the voltages (rate 1 CI8), with the operand ring depth, the raw
+// threads load the voltages (CI8, rates 1 and 2), with the operand ring depth, the raw
 // ring depth and the tiles per raw stage.
 struct TcChoice {
     uint32_t mode, a_stages, r_stages, raw_tiles;
@@ -249,6 +249,10 @@ bool tc_apply(TcShape& s, uint64_t A, uint64_t T, uint32_t es, uint64_t rate, co
     s.smem = s.img_bytes + 1536 + c.a_stages * op + c.r_stages * (size_t)s.raw_bytes;
     return s.smem <= limit;
 }
+
+// Last word of the tuning key of a launch that splits its phasors itself; the plain
+// chain's is the sample size.
+constexpr uint64_t kTuneSelf = 5;
 
 // The launch layout of a chain call: the tuned choice for this shape on this device
 // when blade_beamform_detect_tc_autotune stored one, else the heuristic default.
@@ -335,6 +339,29 @@ bool self_shape(const TcShape& s, uint64_t F, uint64_t T, uint64_t rate, uint32_
     if (per > even + rt) return false;
     segs = (uint32_t)ceil_div(tpc, per);
     seg_tiles = (uint32_t)per;
+    return true;
+}
+
+// The launch layout of a call that splits its phasors inside the chain kernel: the choice
+// tuned for that launch (its operand build and grid are not the plain chain's, so neither's
+// times hold for the other) or the default; false when the default layout is not such a launch.
+bool tc_self_layout(uint64_t B, uint64_t A, uint64_t F, uint64_t T, uint64_t rate, uint64_t integration, TcShape& s,
+                    uint32_t& segs, uint32_t& seg_tiles, bool* tuned = nullptr, TuneEntry* entry = nullptr) {
+    if (tuned) *tuned = false;
+    if (!tc_shape(B, A, s, T, 4, rate) || !self_shape(s, F, T, rate, segs, seg_tiles)) return false;
+    const uint64_t key[8] = {B, A, F, T, 2, rate, integration, kTuneSelf};
+    TuneEntry e;
+    TcShape t = s;
+    uint32_t g, gt;
+    if (tune_lookup(BLADE_TUNE_TC, key, &e) &&
+        tc_apply(t, A, T, 4, rate, TcChoice{e.params[0], e.params[1], e.params[2], e.params[3]}) &&
+        self_shape(t, F, T, rate, g, gt)) {
+        s = t;
+        segs = g;
+        seg_tiles = gt;
+        if (tuned) *tuned = true;
+        if (entry) *entry = e;
+    }
     return true;
 }
 
@@ -514,14 +541,13 @@ extern "C" int blade_beamform_prepare_detect_tc(const void* phasors, void* plan,
     if (F == 0) return BLADE_SUCCESS;  // no split launched: nothing may follow it programmatically
     TcShape s;
     uint32_t segs, seg_tiles;
-    tc_layout(B, A, F, T, rate, integration, 4, s);
-    if (self_shape(s, F, T, rate, segs, seg_tiles))
+    if (tc_self_layout(B, A, F, T, rate, integration, s, segs, seg_tiles))
         return tc_run("blade_beamform_prepare_detect_tc", in, plan, out, B, A, F, T, rate, integration, 4,
                       tc_self_kernel(rate, integration), stream, false, &s, static_cast<const float2*>(phasors), segs,
                       seg_tiles);
     if (int rc = blade_beamform_tc_prepare(phasors, plan, B, A, F, P, stream)) return rc;
     return tc_run("blade_beamform_prepare_detect_tc", in, plan, out, B, A, F, T, rate, integration, 4,
-                  nullptr, stream, true, &s);
+                  nullptr, stream, true);
 }
 
 extern "C" int blade_beamform_detect_tc_cf16(const void* in, const void* plan, void* out, uint64_t B, uint64_t A,
@@ -831,8 +857,12 @@ int tc_query(const uint64_t (&shape)[8], uint32_t* params, float* us, int* tuned
     bool t = false;
     TuneEntry e;
     const uint32_t es = shape[7] ? (uint32_t)shape[7] : 4u;
-    if (shape[4] != 2 || !tc_layout(shape[0], shape[1], shape[2], shape[3], shape[5], shape[6], es, s, &t, &e))
-        return set_error(BLADE_ERROR, "blade_autotune_query: unsupported tensor-core shape");
+    uint32_t segs, seg_tiles;
+    const bool ok = shape[7] == kTuneSelf
+                        ? blade_beamform_detect_tc_supported(shape[0], shape[1], shape[2], shape[3], 2, shape[5], shape[6]) &&
+                              tc_self_layout(shape[0], shape[1], shape[2], shape[3], shape[5], shape[6], s, segs, seg_tiles, &t, &e)
+                        : tc_layout(shape[0], shape[1], shape[2], shape[3], shape[5], shape[6], es, s, &t, &e);
+    if (shape[4] != 2 || !ok) return set_error(BLADE_ERROR, "blade_autotune_query: unsupported tensor-core shape");
     const TcChoice c = tc_choice_of(s);
     for (int i = 0; i < kTuneParams; i++) params[i] = t ? e.params[i] : 0u;
     params[0] = c.mode;
@@ -882,38 +912,51 @@ extern "C" int blade_beamform_detect_tc_autotune(uint64_t B, uint64_t A, uint64_
     for (uint32_t rt : {2u, 1u})
         for (const auto& r : rings) add(TcChoice{0, r[0], r[1], rt});
     for (uint32_t a : {8u, 6u, 4u}) add(TcChoice{1, a, 0, 1});
-    int best = -1;
-    float best_us = 0.f;
-    uint32_t ndiff = 0, ntimed = 0;
-    for (size_t i = 0; i < cands.size(); i++) {
-        TcShape t = base;
-        tc_apply(t, A, T, 4, rate, cands[i]);
-        void* dst = i == 0 ? ref : out;
-        const float us = tune_time(
-            [&]() { return tc_run(who, in, plan, dst, B, A, F, T, rate, integration, 4, nullptr, stream, false, &t); }, st);
-        if (us < 0.f) return set_error(BLADE_CUDA_ERROR, "%s: candidate %zu failed: %s", who, i, blade_last_error());
-        uint32_t status = 0;
-        if (int rc = blade_device_status(&status)) return rc;
-        if (status != 0) return set_error(BLADE_CUDA_ERROR, "%s: candidate %zu: device status %u", who, i, status);
-        ntimed++;
-        if (i > 0 && !tune_same(ref, out, out_bytes)) {
-            ndiff++;
-            continue;
+    // The plain chain, then, for a block whose prepared call splits its phasors inside the
+    // chain kernel, that launch.
+    uint32_t segs, seg_tiles;
+    const bool small = self_shape(base, F, T, rate, segs, seg_tiles);
+    for (int self = 0; self <= (small ? 1 : 0); self++) {
+        int best = -1;
+        float best_us = 0.f;
+        uint32_t ndiff = 0, ntimed = 0;
+        for (size_t i = 0; i < cands.size(); i++) {
+            TcShape t = base;
+            tc_apply(t, A, T, 4, rate, cands[i]);
+            if (self && !self_shape(t, F, T, rate, segs, seg_tiles)) continue;
+            void* dst = i == 0 ? ref : out;
+            const float us = tune_time(
+                [&]() {
+                    return self ? tc_run(who, in, plan, dst, B, A, F, T, rate, integration, 4,
+                                         tc_self_kernel(rate, integration), stream, false, &t,
+                                         static_cast<const float2*>(ph), segs, seg_tiles)
+                                : tc_run(who, in, plan, dst, B, A, F, T, rate, integration, 4, nullptr, stream, false, &t);
+                },
+                st);
+            if (us < 0.f) return set_error(BLADE_CUDA_ERROR, "%s: candidate %zu failed: %s", who, i, blade_last_error());
+            uint32_t status = 0;
+            if (int rc = blade_device_status(&status)) return rc;
+            if (status != 0) return set_error(BLADE_CUDA_ERROR, "%s: candidate %zu: device status %u", who, i, status);
+            ntimed++;
+            if (i > 0 && !tune_same(ref, out, out_bytes)) {
+                ndiff++;
+                continue;
+            }
+            if (best < 0 || us < best_us) {
+                best = (int)i;
+                best_us = us;
+            }
         }
-        if (best < 0 || us < best_us) {
-            best = (int)i;
-            best_us = us;
-        }
+        TuneEntry e = {};
+        e.params[0] = cands[best].mode;
+        e.params[1] = cands[best].a_stages;
+        e.params[2] = cands[best].r_stages;
+        e.params[3] = cands[best].raw_tiles;
+        e.params[4] = ntimed;
+        e.params[5] = ndiff;
+        e.us = best_us;
+        const uint64_t key[8] = {B, A, F, T, P, rate, integration, self ? kTuneSelf : 4};
+        tune_store(BLADE_TUNE_TC, key, e);
     }
-    TuneEntry e = {};
-    e.params[0] = cands[best].mode;
-    e.params[1] = cands[best].a_stages;
-    e.params[2] = cands[best].r_stages;
-    e.params[3] = cands[best].raw_tiles;
-    e.params[4] = ntimed;
-    e.params[5] = ndiff;
-    e.us = best_us;
-    const uint64_t key[8] = {B, A, F, T, P, rate, integration, 4};
-    tune_store(BLADE_TUNE_TC, key, e);
     return BLADE_SUCCESS;
 }

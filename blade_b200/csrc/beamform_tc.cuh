@@ -107,7 +107,7 @@ struct TcArgs {
     uint32_t raw_tiles, raw_row;  // tiles per raw stage (1, 2 or 4) and its antenna row stride (raw_tiles * 512)
     uint64_t total_tiles;
     uint32_t pdl;  // launched as a programmatic dependent of the phasor split: wait for it before the image
-    uint32_t direct;  // R = 1 CI8 without a raw ring: converter threads load the voltages themselves
+    uint32_t direct;  // CI8 at R = 1 or 2 without a raw ring: converter threads load the voltages themselves
     uint32_t transposed;  // outputs along TMEM lanes, samples along columns (64-beam chunks, rate 1, I = 8 or 16)
     const float2* ph;      // SELF: the chunk's phasors [beams][A][F][2]
     uint8_t* plan_out;     // SELF: where the images go besides

@@ -402,8 +402,9 @@ BLADE_API int blade_source_direction(double ra, double dec, double julian_date, 
  *   BLADE_TUNE_TC (blade_beamform_detect_tc, blade_beamform_prepare_detect_tc,
  *     blade_beamform_detect_tc_noalloc): key {B, A, F, T, P, rate, integration, 4};
  *     params {mode (0 raw ring of TMA tiles, 1 converter threads load the
- *     voltages, 2 phasor rows in tensor memory), operand stages, raw stages,
- *     tiles per raw stage}.
+ *     voltages), operand stages, raw stages, tiles per raw stage}.  On small blocks the
+ *     prepared and the no-alloc call split their phasors inside the chain kernel, a
+ *     launch that is timed and stored separately, with 5 as the key's last word.
  *   BLADE_TUNE_F32 (blade_beamform_detect_f32): key {B, A, F, T, P, rate,
  *     integration, in_type}; params {time-group width TG (a CTA covers 4 TG
  *     samples and 1024 / TG beams), 0, 0, 0}.
