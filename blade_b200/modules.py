@@ -868,12 +868,18 @@ class ModeH(Module):
         return result.success
 
 
+def _aligned(buffer, nbytes: int) -> bool:
+    """Whether every slot of a module's input starts on a multiple of `nbytes`."""
+    slots = [buffer.at(0), buffer.at(1)] if isinstance(buffer, Duet) else [buffer]
+    return all(v.data_ptr() % nbytes == 0 for v in slots)
+
+
 class _ModeBTensorCore(Module):
     """ModeB on CI8 voltages with the detector (Stokes-I) at channelizer rate 2 or 4,
     on tensor cores with per-fine-channel phasors.
 
     direct (blade_modeb_detect_tc: up to 32 antennas, 16 beams at rate 4 or 32 at
-    rate 2): the phasor split and one chain from the CI8 block, which transforms and
+    rate 2, 16-byte aligned voltages): the phasor split and one chain from the CI8 block, which transforms and
     polarizes while it builds its operand; the detected incoherent beam, when
     enabled, also comes from the CI8 block (blade_incoherent_detect_ci8).
     Otherwise the pre-beamformer stages go to an exact CF16 buffer
@@ -890,7 +896,7 @@ class _ModeBTensorCore(Module):
         A, F, T, P = as_vector(buffer).shape
         B = as_vector(phasors).shape[0]
         R = self._R
-        self.direct = self._direct(A, F, T, P, B, R, self._I)
+        self.direct = _aligned(buffer, 16) and self._direct(A, F, T, P, B, R, self._I)
         self._pre = None if self.direct else self._alloc((A, F * R, T // R, P), "cf16")
         n = int(_lib.load().blade_beamform_tc_plan_size(B, A, F * R, P))
         self._plan = self._alloc((n,), "i8", "tensor")
@@ -1105,9 +1111,11 @@ class ModeB(Module):
             circ, inc = bool(c.pre_beamformer_polarizer_convert_to_circular), bool(c.beamformer_incoherent_beam)
             products = (bool(c.detector_enable) and OP in (1, 4) and R >= 1 and T % R == 0
                         and _BeamformProducts.applies(A, F * R, T // R, P, B, I, OP))
-            if R == 1 and not circ and P == 2 and (products or it == "cf32"):
+            # the launches that read CI8 take whole samples, the Cast any alignment
+            samples = it == "cf32" or _aligned(input.buffer, 4)
+            if R == 1 and not circ and P == 2 and samples and (products or it == "cf32"):
                 voltages = input.buffer
-            elif _ModeBPre.applies(it, T, P, R):
+            elif samples and _ModeBPre.applies(it, T, P, R):
                 pre = _ModeBPre(input.buffer, R, circ)
                 voltages = pre.get_output()
                 self._stages.append(pre)
