@@ -1135,8 +1135,7 @@ __global__ void __launch_bounds__(kThreads, 1) bf_tc_kernel(const TcArgs g, cons
                     tc_fence_after();
                     if (lane == 0) {
                         const uint64_t ad = a_desc + (uint64_t)((as + j) * op16), wd = w_desc + (uint64_t)(j * R * wpol16);
-                        if (KA == 64) issue_stacked<8>(tmem + j * d_cols, ad, wd, 4 * R * nb16, idesc);
-                        else issue_stacked<4>(tmem + j * d_cols, ad, wd, 4 * R * nb16, idesc);
+                        issue_stacked<4>(tmem + j * d_cols, ad, wd, 4 * R * nb16, idesc);  // KA = 32
                         mma_commit(&a_empty[as + 1]);
                         mma_commit(&d_full[j]);
                     }
