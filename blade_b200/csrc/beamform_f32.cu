@@ -247,26 +247,35 @@ __global__ void __launch_bounds__(256, 2) bf32_kernel(const void* __restrict__ v
 // polarisations, antennas in order, nothing staged.  Bound by latency: the loads of a few
 // antennas are in flight at a time and every beam re-reads the voltages from L2.  Same
 // arithmetic per output as the streaming kernel.
+struct SmallArgs {
+    uint32_t A, F, T;
+    PhLayout ph;
+    // 96 bytes of kernel parameters: a launch with 72 or 80 takes 0.6 us longer on the host.
+    // (Aligning the struct instead moves its fields, and the one-polarisation loop takes 5 to
+    // 10 % longer.)
+    uint64_t pad[3];
+};
+
 template <int P>
 __global__ void __launch_bounds__(256) bf32_small_kernel(const float2* __restrict__ in,
                                                          const float2* __restrict__ phasors, float2* __restrict__ out,
-                                                         uint32_t A, uint32_t F, uint32_t T, const PhLayout ph) {
+                                                         const SmallArgs g) {
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x, f = blockIdx.y, b = blockIdx.z;
-    if (t >= T) return;
+    if (t >= g.T) return;
     float2 acc[P];
 #pragma unroll
     for (int p = 0; p < P; p++) acc[p] = make_float2(0.f, 0.f);
-    const float2* x = in + ((uint64_t)f * T + t) * P;
-    const float2* w = phasors + b * ph.sb + (uint64_t)f * ph.sf;
-    for (uint32_t a = 0; a < A; a++) {
+    const float2* x = in + ((uint64_t)f * g.T + t) * P;
+    const float2* w = phasors + b * g.ph.sb + (uint64_t)f * g.ph.sf;
+    for (uint32_t a = 0; a < g.A; a++) {
 #pragma unroll
         for (int p = 0; p < P; p++) {
-            const float2 xv = __ldg(x + (uint64_t)a * F * T * P + p), wv = __ldg(w + a * ph.sa + p * ph.sp);
+            const float2 xv = __ldg(x + (uint64_t)a * g.F * g.T * P + p), wv = __ldg(w + a * g.ph.sa + p * g.ph.sp);
             acc[p].x = fmaf(xv.x, wv.x, fmaf(-xv.y, wv.y, acc[p].x));
             acc[p].y = fmaf(xv.x, wv.y, fmaf(xv.y, wv.x, acc[p].y));
         }
     }
-    float2* o = out + (((uint64_t)b * F + f) * T + t) * P;
+    float2* o = out + (((uint64_t)b * g.F + f) * g.T + t) * P;
 #pragma unroll
     for (int p = 0; p < P; p++) o[p] = acc[p];
 }
@@ -319,19 +328,21 @@ int launch_stream_beams(const StreamArgs& g, uint32_t nb, uint32_t ns, cudaStrea
 // Whether bf32_small_kernel takes a block: its launch has no ring to fill and no weights to
 // gather, which is worth 0.2 to 0.7 us while its CTAs are resident at once.
 //   Two polarisations: up to 4 antennas (192 samples, 8 beams: 1.8 us against 2.2 streamed),
-//   up to 8 at half of the warps an SM holds (2.0 against 2.5; one beam 4.9 against 5.4 at all
-//   of them); with 16 the antennas' serial loads already cost more (0.73 to 0.99 of its time
-//   streamed).
+//   up to 6 at half of the warps an SM holds, up to 8 for one beam at more (4.9 against 5.4);
+//   with 16 the antennas' serial loads already cost more (0.73 to 0.99 of its time streamed).
 //   One polarisation: half of the warps and 48 MB of voltages, which stay in L2 for the beams
 //   that re-read them (1.0 to 1.3 times the speed at 96 to 256 antennas; at 60 MB and more
-//   the ring is up to 1.6 times ahead), and one beam, which re-reads none, at more warps than
-//   that (64 antennas x 192 x 1024: 14.0 us against 17.4; 1024 antennas: 243 against 286).
+//   the ring is up to 1.6 times ahead).  One beam re-reads none: 72 MB (192 antennas, 72 MB:
+//   13.6 us against 15.1; 256 antennas, 96 MB: 41 against 29), any amount at more warps than
+//   that (64 antennas x 192 x 1024: 14.0 against 17.4; 1024 antennas: 243 against 286), and
+//   beyond 64 antennas at least four warps per SM (160 antennas, 256 samples: 10.8 against 9.8).
 bool small_shape(uint64_t B, uint64_t A, uint64_t F, uint64_t T, uint64_t P) {
     const uint64_t sms = (uint64_t)sm_count(), warps = B * F * ceil_div(T, 32);
     if (B * F * ceil_div(T, 256) > 8 * sms) return false;
     const bool half = warps <= 32 * sms;
-    if (P == 2) return A <= (B == 1 ? 8 : 4) || (A <= 8 && half);
-    return A <= 4 || (half ? A * F * T * sizeof(float2) <= 48u << 20 : B == 1);
+    if (P == 2) return A <= (half ? 6 : B == 1 ? 8 : 4);
+    if (!half) return A <= 4 || B == 1;
+    return A * F * T * sizeof(float2) <= (B == 1 ? 72u : 48u) << 20 && (B > 1 || A <= 64 || warps > 4 * sms);
 }
 
 // Beams 0..B-1 of the plain FP32 beamformer for a phasor layout, and with inc the
@@ -341,9 +352,11 @@ int beamform_f32_beams(const char* who, const void* in, const float2* ph, void* 
     if (B == 0) return BLADE_SUCCESS;
     if (!inc && small_shape(B, A, F, T, P)) {
         const dim3 grid((unsigned)ceil_div(T, 256), (unsigned)F, (unsigned)B);
-        const auto fn = P == 2 ? bf32_small_kernel<2> : bf32_small_kernel<1>;
-        fn<<<grid, 256, 0, s>>>(static_cast<const float2*>(in), ph, static_cast<float2*>(out), (uint32_t)A,
-                                (uint32_t)F, (uint32_t)T, lay);
+        const SmallArgs g{(uint32_t)A, (uint32_t)F, (uint32_t)T, lay};
+        const float2* x = static_cast<const float2*>(in);
+        float2* y = static_cast<float2*>(out);
+        if (P == 2) bf32_small_kernel<2><<<grid, 256, 0, s>>>(x, ph, y, g);
+        else bf32_small_kernel<1><<<grid, 256, 0, s>>>(x, ph, y, g);
         return check_launch(who);
     }
     uint32_t nb, ns;

@@ -26,6 +26,8 @@
 // the detector.
 #pragma once
 
+#include <type_traits>
+
 #include "common.cuh"
 
 namespace bb {
@@ -46,9 +48,12 @@ struct StreamArgs {
     uint32_t inc;        // 0 none, 1 sum of powers, 2 its square root
     uint32_t nbt;        // beam tiles, innermost in the grid (they read the same voltages)
     uint32_t ntt;        // time tiles per channel
-    uint32_t chunk;      // antennas whose weights are in shared memory at a time
     uint64_t tiles;      // F * ntt
     PhLayout lay;
+};
+
+struct StreamChunkArgs : StreamArgs {
+    uint32_t chunk;  // antennas whose weights are in shared memory at a time
 };
 
 constexpr int kStreamWarps = 4;
@@ -88,7 +93,7 @@ struct StreamSample {
 // of spills at eight beams and two samples).
 template <int P, int NB, int NS, int IN, int OP, bool CHUNKED>
 __global__ void __launch_bounds__(kStreamWarps * 32, NB == 8 && NS == 2 ? (CHUNKED ? 4 : 5) : 1)
-    bf_stream_kernel(const StreamArgs g) {
+    bf_stream_kernel(const std::conditional_t<CHUNKED, StreamChunkArgs, StreamArgs> g) {
     using Sample = StreamSample<P, IN>;
     constexpr uint32_t kThreads = kStreamWarps * 32, kSlot = kThreads * Sample::kBytes;
     extern __shared__ __align__(16) unsigned char stream_smem_raw[];  // ring [kStreamDepth][NS][thread], weights
@@ -121,23 +126,21 @@ __global__ void __launch_bounds__(kStreamWarps * 32, NB == 8 && NS == 2 ? (CHUNK
 #pragma unroll
     for (uint32_t a = 0; a < kStreamDepth - 1; a++)  // on their way while the weights are gathered
         fetch(a, ring + a * NS * kSlot);
-    // weights of this CTA's channels and of antennas a0 to a1, padded beams zero
-    const uint32_t held = CHUNKED ? g.chunk : g.A;
-    auto gather = [&](uint32_t a0, uint32_t a1) {
-#pragma unroll 4
-        for (uint32_t r = tid; r < NB * (a1 - a0); r += kThreads) {
-            const uint32_t a = r / NB, j = r - a * NB;
-            const bool ok = b0 + j < g.B;
-            const float2* wsrc = g.ph + (b0 + j) * g.lay.sb + (a0 + a) * g.lay.sa + (uint64_t)f0 * g.lay.sf;
-            for (uint32_t c = 0; c < nch; c++)
+    // weight r of this CTA's channels and of the antennas held from a0 on, padded beams zero
+    uint32_t held = g.A;
+    if constexpr (CHUNKED) held = g.chunk;
+    auto gather = [&](uint32_t r, uint32_t a0) {
+        const uint32_t a = r / NB, j = r - a * NB;
+        const bool ok = b0 + j < g.B;
+        const float2* wsrc = g.ph + (b0 + j) * g.lay.sb + (a0 + a) * g.lay.sa + (uint64_t)f0 * g.lay.sf;
+        for (uint32_t c = 0; c < nch; c++)
 #pragma unroll
-                for (int p = 0; p < P; p++)
-                    ws[((c * held + a) * NB + j) * P + p] = ok ? __ldg(wsrc + c * g.lay.sf + p * g.lay.sp) : make_float2(0.f, 0.f);
-        }
-        __syncthreads();
+            for (int p = 0; p < P; p++)
+                ws[((c * held + a) * NB + j) * P + p] = ok ? __ldg(wsrc + c * g.lay.sf + p * g.lay.sp) : make_float2(0.f, 0.f);
     };
     if constexpr (!CHUNKED) {
-        gather(0, g.A);
+        for (uint32_t r = tid; r < NB * g.A; r += kThreads) gather(r, 0);
+        __syncthreads();
         if (!active) {
             asm volatile("cp.async.wait_all;" ::: "memory");
             return;
@@ -196,10 +199,11 @@ __global__ void __launch_bounds__(kStreamWarps * 32, NB == 8 && NS == 2 ? (CHUNK
         for (uint32_t a = 0; a < g.A; a++) antenna(a);
     } else {
 #pragma unroll 1
-        for (uint32_t a0 = 0; a0 < g.A; a0 += g.chunk) {
-            const uint32_t a1 = min(a0 + g.chunk, g.A);
+        for (uint32_t a0 = 0; a0 < g.A; a0 += held) {
+            const uint32_t a1 = min(a0 + held, g.A);
             if (a0) __syncthreads();  // every warp has read the chunk before
-            gather(a0, a1);
+            for (uint32_t r = tid; r < NB * (a1 - a0); r += kThreads) gather(r, a0);
+            __syncthreads();
             if (!active) continue;
             wa = ws + (size_t)(f - f0) * held * NB * P;
 #pragma unroll 1
@@ -311,12 +315,21 @@ int launch_stream(StreamArgs g, cudaStream_t s) {
     // whole, 957 in chunks (1357 for 4 x 4 register tiles staged behind a barrier); 2048 antennas,
     // 64 channels, 64 beams: 7920, 3430 (and 4057).
     const size_t room = 224 * 1024 / (per_sm < 4 ? per_sm : 4) - ring;
-    const bool chunked = g.A * antenna > room;
-    g.chunk = chunked ? (uint32_t)(room / antenna) : g.A;
-    const size_t smem = ring + g.chunk * antenna;
-    const auto fn = chunked ? bf_stream_kernel<P, NB, NS, IN, OP, true> : bf_stream_kernel<P, NB, NS, IN, OP, false>;
+    const unsigned grid = (unsigned)ctas, block = kStreamWarps * 32;
+    if (g.A * antenna <= room) {
+        const auto fn = bf_stream_kernel<P, NB, NS, IN, OP, false>;
+        const size_t smem = ring + g.A * antenna;
+        if (int rc = ensure_smem(reinterpret_cast<const void*>(fn), smem)) return rc;
+        fn<<<grid, block, smem, s>>>(g);
+        return BLADE_SUCCESS;
+    }
+    StreamChunkArgs h;
+    static_cast<StreamArgs&>(h) = g;
+    h.chunk = (uint32_t)(room / antenna);
+    const auto fn = bf_stream_kernel<P, NB, NS, IN, OP, true>;
+    const size_t smem = ring + h.chunk * antenna;
     if (int rc = ensure_smem(reinterpret_cast<const void*>(fn), smem)) return rc;
-    fn<<<(unsigned)ctas, kStreamWarps * 32, smem, s>>>(g);
+    fn<<<grid, block, smem, s>>>(h);
     return BLADE_SUCCESS;
 }
 
