@@ -653,10 +653,10 @@ __global__ void __launch_bounds__(kPairThreads8, 1) fft8192_pair_kernel(const fl
 //
 // Bound by instruction issue and the shared-memory exchanges (blocks whose workspace
 // stays in L2 take as long per channel): the spectrometer's 64 channels x 16
-// spectra (CI8 in, windows of 8) 531 us for 2.45 GB (4.6 TB/s), 796 us for one
+// spectra (CI8 in, windows of 8) 541 to 553 us for 2.45 GB (4.5 TB/s), 796 us for one
 // transform per thread group with three shared-memory passes per step and twiddle
-// recurrences.  The next group's input is asked for while a group is transformed (551 us
-// without); three CTAs per SM spill and take 730 us.  Error against 64 bits 1.5e-7
+// recurrences.  The next group's input is asked for while a group is transformed (20 us
+// longer without); three CTAs per SM spill and take 730 us.  Error against 64 bits 1.5e-7
 // where the recurrences gave 4.2e-7.
 constexpr uint32_t k65Threads = 256;
 constexpr uint32_t k65Ld = 257;  // pairs per unit in the row step's exchange
