@@ -164,10 +164,10 @@ __device__ __forceinline__ float4 circular_f4(float4 v) {
     return make_float4(v.x - v.w, v.y + v.z, v.x + v.w, v.y - v.z);
 }
 
-template <int P, bool CI8>
+template <int P, bool CI8, bool CIRC>
 __global__ void __launch_bounds__(kThreads) fft_small_kernel(const void* __restrict__ vin, float2* __restrict__ out,
                                                              uint32_t A, uint32_t F, uint32_t T, uint32_t N,
-                                                             uint32_t SB, Plan plan, int circular) {
+                                                             uint32_t SB, Plan plan) {
     extern __shared__ __align__(16) float2 smem[];
     const uint32_t S = T / N;
     const uint32_t G = SB * P;
@@ -209,7 +209,7 @@ __global__ void __launch_bounds__(kThreads) fft_small_kernel(const void* __restr
             if (P == 2) {
                 const float2 x0 = res[(sl * 2 + 0) * N + kk], x1 = res[(sl * 2 + 1) * N + kk];
                 const float4 v = make_float4(x0.x, x0.y, x1.x, x1.y);
-                stg_f4(dst, circular ? circular_f4(v) : v);
+                stg_f4(dst, CIRC ? circular_f4(v) : v);
             } else {
                 dst[0] = res[sl * N + kk];
             }
@@ -926,15 +926,18 @@ int channelize_small(const char* who, const void* in, bool ci8, float2* out, uin
     const size_t smem = (rate + 2 * SB * P * rate) * sizeof(float2);
     const uint64_t groups = rows * ceil_div(S, SB), cap = (uint64_t)sm_count() * 2;
     const unsigned grid = (unsigned)(groups < cap ? groups : cap);
-#define BB_FFT_SMALL(PP, C8)                                                                                   \
-    do {                                                                                                       \
-        if (int rc = prepare_smem(fft_small_kernel<PP, C8>, smem)) return rc;                                  \
-        fft_small_kernel<PP, C8><<<grid, kThreads, smem, s>>>(in, out, (uint32_t)A, (uint32_t)F, (uint32_t)T,  \
-                                                              (uint32_t)rate, (uint32_t)SB, plan, circular);   \
+#define BB_FFT_SMALL(PP, C8, CC)                                                                              \
+    do {                                                                                                      \
+        if (int rc = prepare_smem(fft_small_kernel<PP, C8, CC>, smem)) return rc;                             \
+        fft_small_kernel<PP, C8, CC><<<grid, kThreads, smem, s>>>(in, out, (uint32_t)A, (uint32_t)F,          \
+                                                                  (uint32_t)T, (uint32_t)rate, (uint32_t)SB,  \
+                                                                  plan);                                      \
     } while (0)
-    if (ci8) BB_FFT_SMALL(2, true);
-    else if (P == 2) BB_FFT_SMALL(2, false);
-    else BB_FFT_SMALL(1, false);
+    if (ci8 && circular) BB_FFT_SMALL(2, true, true);
+    else if (ci8) BB_FFT_SMALL(2, true, false);
+    else if (P == 2 && circular) BB_FFT_SMALL(2, false, true);
+    else if (P == 2) BB_FFT_SMALL(2, false, false);
+    else BB_FFT_SMALL(1, false, false);
 #undef BB_FFT_SMALL
     return check_launch(who);
 }
