@@ -22,7 +22,10 @@
 // Bound by HBM: 8 antennas x 192 channels x 8192 samples, two polarisations (403 MB
 // in and out): 70 us at rates 32, 64 and 256 (5.7 TB/s), 73 at 128, 78 at 1024, 89 at
 // 512, 112 at 4096 (one unit per CTA there: 16-byte runs), against 263 to 470 us for
-// passes of radix 8 and 4 through shared memory on one transform at a time.
+// passes of radix 8 and 4 through shared memory on one transform at a time.  The radix-16
+// stages carry their constants to twice FP32's precision (0 to 2 % of that, 4 to 6 on blocks
+// that stay in L2): rounded, two of them put 5.3e-8 on the mean power at rate 256 and three
+// 7.7e-8 at 4096, where passes of radix 8 and 4 gave 4.0e-8 and 5.7e-8; now 0.7e-8 and 0.9e-8.
 #include "channelize.cuh"
 #include "fft_regs.cuh"
 
@@ -89,7 +92,7 @@ __global__ void __launch_bounds__(kPowThreads, R1 == 16 ? 2 : 3)
                     v[m] = c2{make_float2(a.x, b.x), make_float2(a.y, b.y)};
                 }
             }
-            dft<R1>(v);
+            dft<R1, true>(v);
             twiddle_column<R1>(v, tw1 + t, M1);
 #pragma unroll
             for (int k1 = 0; k1 < R1; k1++) put(u * LDs + k1 * LD1 + t, v[k1]);
@@ -102,7 +105,7 @@ __global__ void __launch_bounds__(kPowThreads, R1 == 16 ? 2 : 3)
                 c2 v[R2];
 #pragma unroll
                 for (int i = 0; i < R2; i++) v[i] = get(base + i * R3);
-                dft<R2>(v);
+                dft<R2, true>(v);
                 twiddle_column<R2>(v, tw2 + x, R3);
 #pragma unroll
                 for (int k2 = 0; k2 < R2; k2++) put(base + k2 * R3, v[k2]);
@@ -118,7 +121,7 @@ __global__ void __launch_bounds__(kPowThreads, R1 == 16 ? 2 : 3)
             c2 v[RL];
 #pragma unroll
             for (int i = 0; i < RL; i++) v[i] = get(base + i);
-            dft<RL>(v);
+            dft<RL, true>(v);
 #pragma unroll
             for (int k3 = 0; k3 < RL; k3++) {
                 const uint32_t kout = (q + (N / RL) * k3 + N / 2) & (N - 1);  // fftshift; q = k1 + R1 k2
